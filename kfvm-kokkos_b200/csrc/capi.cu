@@ -276,12 +276,15 @@ struct kfvm_solver {
   void *xuser = nullptr;
   double *xbuf[4] = {nullptr, nullptr, nullptr, nullptr};
   // TMA maps of the three state buffers for the tensor-core reconstruction's halo
-  // tiles (built when the FP32 form is selected; unused where the pitch is odd)
+  // tiles (built when the FP32 form is selected)
   CUtensorMap umap[3];
   bool umapOk = false;
-  // and those of the FP64 reconstruction's halo tiles (five variables or 2D, even pitch)
+  // and those of the FP64 reconstruction's state tiles (with three Gauss points: five
+  // variables in 2D only), and its parity weights (two Gauss points, not SR)
   CUtensorMap dmap[3];
   bool dmapOk = false;
+  kfvm::SymW symw;
+  bool symOk = false;
   int64_t nRhs = 0, nWenoLast = 0;
   int nTS = 1;
   double dmin = 0.0;
@@ -556,9 +559,13 @@ int eval_front(kfvm_solver *s, int b) {
              // the limiter bounds of every cell, then the linear states
              cudaError_t eb = launch_bounds(dim, eq, s->Ub[b], s->g, s->bnd, st);
              if (eb != cudaSuccess) return eb;
-             return launch_recon_tc(dim, eq, s->Ub[b], s->umapOk ? &s->umap[b] : nullptr, s->g, s->dS, wantInd,
+             return launch_recon_tc(dim, eq, s->Ub[b], s->umap[b], s->g, s->dS, wantInd,
                                     s->F, s->W, s->src, s->status,
                                     s->lamvel, s->bnd, s->sc, st);
+           }
+           if (s->symOk) {
+             const ReconSymArgs a{wantInd, s->F, s->W, s->src, s->status, s->lamvel, s->bnd, s->sc};
+             return launch_recon_sym(dim, eq, a, s->dmap[b], s->g, s->symw, st);
            }
            return launch_recon(dim, eq, s->Ub[b], s->dmapOk ? &s->dmap[b] : nullptr, s->g, s->dS, wantInd, s->F,
                                s->W, s->src, s->status, s->lamvel, s->bnd, s->sc, st);
@@ -927,7 +934,8 @@ int kfvm_create(const kfvm_config *cfg, kfvm_solver **out) {
   g.ny = cfg->ny;
   g.nz = nz;
   g.n = g.nx * g.ny * g.nz;
-  g.px = g.nx + 2 * kRad;
+  // an even row pitch: the strides of the state's tensor maps are multiples of 16 bytes
+  g.px = (g.nx + 2 * kRad + 1) & ~(int64_t)1;
   g.py = g.ny + 2 * kRad;
   g.rz = cfg->dim == 3 ? kRad : 0;
   g.pvol = g.px * g.py * (cfg->dim == 3 ? nz + 2 * kRad : 1);
@@ -981,7 +989,12 @@ int kfvm_create(const kfvm_config *cfg, kfvm_solver **out) {
         for (int q = 0; q < hS.w.nqc; q++) hS.lin[c * nrows + r++] = hS.w.cell_w[0][q][c];
     }
     if (cfg->nq == 2) fill_tc_weights(hS, cfg->dim, nrows);  // the tensor-core form takes 2 points only
-    fill_dmma_weights(hS, nrows);
+    s->symOk = cfg->nq == 2 && cfg->eq != KFVM_EQ_SRHYDRO;
+    if (!s->symOk) fill_dmma_weights(hS, nrows);
+  }
+  if (s->symOk && fill_sym_weights(hS.w, cfg->eq == KFVM_EQ_MHD_GLM, s->symw) != 0) {
+    delete s;
+    return fail(KFVM_ERR_ARG, "the reconstruction weights of mirrored points are not mirror images");
   }
 
   auto cleanup = [&](cudaError_t e, const char *what) {
@@ -1045,12 +1058,17 @@ int kfvm_create(const kfvm_config *cfg, kfvm_solver **out) {
   if ((e = cudaMemsetAsync(s->sc, 0, sizeof(DevScalars), s->stream)) != cudaSuccess) return cleanup(e, "memset");
 
   if ((e = cudaStreamSynchronize(s->stream)) != cudaSuccess) return cleanup(e, "sync");
-  // TMA maps of the FP64 reconstruction's halo tiles (five variables, or GLM-MHD in
-  // 2D; even pitch; otherwise that kernel reads the state with plain loads)
-  if (s->nv == 5 || s->dim == 2) {
+  // TMA maps of the FP64 reconstruction's state tiles
+  if (s->symOk || (s->nv == 5 && (s->dim == 2 || cfg->eq == KFVM_EQ_SRHYDRO))) {
     bool all = true;
-    for (int b = 0; b < 3; b++) all = all && recon_dmma_state_map(&s->dmap[b], s->Ub[b], g, s->dim, s->nv) == 0;
+    for (int b = 0; b < 3; b++)
+      all = all && (s->symOk ? recon_sym_state_map(&s->dmap[b], s->Ub[b], g, s->dim, s->nv)
+                              : recon_dmma_state_map(&s->dmap[b], s->Ub[b], g, s->dim, s->nv)) == 0;
     s->dmapOk = all;
+    if (s->symOk && !all) {
+      kfvm_destroy(s);
+      return fail(KFVM_ERR_CUDA, "the tensor maps of the state buffers could not be encoded");
+    }
   }
   *out = s;
   return KFVM_OK;
@@ -1241,7 +1259,8 @@ int kfvm_set_precision(kfvm_solver *s, int32_t precision) {
       bool all = true;
       for (int b = 0; b < 3; b++)
         all = all && kfvm::recon_tc_state_map(&s->umap[b], s->Ub[b], s->g, s->dim, s->nv) == 0;
-      s->umapOk = all;
+      if (!all) return fail(KFVM_ERR_CUDA, "the tensor maps of the state buffers could not be encoded");
+      s->umapOk = true;
     }
   }
   s->precision = precision;

@@ -512,10 +512,8 @@ __global__ void __launch_bounds__(DmmaTile<DIM>::THREADS, (DIM == 2 && NQ == 2 &
 }
 
 // host: the 4D tensor map of a padded state buffer for the TMA-staged tiles (x, y,
-// z, variable; box = the halo tile of one variable).  Returns nonzero where TMA
-// cannot be used (an odd pitch breaks the 16-byte stride rule).
+// z, variable; box = the halo tile of one variable)
 int recon_dmma_state_map(CUtensorMap *map, const double *U, const Grid &g, int dim, int nv) {
-  if (g.px % 2 != 0) return 1;
   const uint64_t planes = (uint64_t)(g.pvol / (g.px * g.py));
   const uint64_t dims[4] = {(uint64_t)g.px, (uint64_t)g.py, planes, (uint64_t)nv};
   const uint64_t strides[3] = {(uint64_t)g.px * 8, (uint64_t)(g.px * g.py) * 8, (uint64_t)g.pvol * 8};
@@ -2118,7 +2116,9 @@ struct Launch {
   static cudaError_t recon(const double *U, const CUtensorMap *umap, const Grid &g, const DevStencil *S,
                            int wantInd, double *const *F, float *const *W, double *src, uint8_t *status,
                            double2 *lamvel, double *bnd, DevScalars *sc, cudaStream_t s) {
-    if constexpr (DmmaShape<DIM, EQ, NQ>::NT > 7) {
+    if constexpr (NQ == 2 && EQ != EQ_SR) {
+      return cudaErrorInvalidValue;  // launch_recon_sym
+    } else if constexpr (DmmaShape<DIM, EQ, NQ>::NT > 7) {
       // more rows than the DMMA kernels hold (3D GLM-MHD, three points)
       using R = RowsShape<DIM, EQ, NQ>;
       static const cudaError_t attrR = cudaFuncSetAttribute(
@@ -2128,13 +2128,11 @@ struct Launch {
           U, g, S, wantInd, F[0], F[1], F[2], W[0], W[1], W[2], src, status, lamvel, bnd);
       return cudaGetLastError();
     } else {
-    // (3D with three Gauss points keeps the global-load kernel: its 54 rows need
-    // more accumulator registers than two 256-thread blocks per SM leave; so does
-    // GLM-MHD in 3D, whose nine halo tiles would not leave room for two blocks, and
-    // with three points in 2D)
-    if constexpr ((NV == 5 && (DIM == 2 || NQ == 2)) || (NV == 9 && DIM == 2 && NQ == 2)) {
+    // (in 3D the 54 rows need more accumulator registers than two 256-thread blocks
+    // per SM leave, and so do GLM-MHD's nine variables in 2D: plain global loads)
+    if constexpr (NV == 5 && (DIM == 2 || EQ == EQ_SR)) {
       if (umap) {
-        // the halo tiles staged by TMA (five variables: Euler, Navier-Stokes, SR)
+        // the halo tiles staged by TMA (Euler, Navier-Stokes, SR)
         using D = DmmaTile<DIM>;
         using L = DmmaTmaSmem<DIM, EQ, NQ>;
         static const cudaError_t attr = cudaFuncSetAttribute(

@@ -4,8 +4,9 @@
 //   bc_fill      periodic / outflow halo of the stage state   (Solver::setCellBCs)
 //   recon        linear face states of every cell written to the face arrays, the
 //                KXRCF indicator at each own face point and whether every state lies
-//                inside the positivity bounds (KernelLinearRecon_K); FP64 FMAs, or
-//                the 3xTF32 tcgen05 contraction of recon_tc.cu
+//                inside the positivity bounds (KernelLinearRecon_K); FP64 by parity
+//                (recon_sym.cu), the direct FP64 sum for three Gauss points and SR
+//                (kernels.cu), or the 3xTF32 tcgen05 contraction of recon_tc.cu
 //   flag         KXRCF flags from the indicators               (WenoSelect_K)
 //   compact      the flag-set semantics of WenoSelector::update, theta = 1 for
 //                in-bounds linear cells, the compacted list of heavy cells
@@ -78,6 +79,14 @@ struct DevStencil {
   double lin[KFVM_MAX_CELLS * kMaxLinRows];
   alignas(16) float tcw[2][kTcMaxK * kTcMaxN];
   alignas(16) double dmma_b[kDmmaMaxB];
+};
+
+// The full-stencil weights for two Gauss points by parity (recon_sym.cu): the point
+// groups x faces, y faces, (z faces,) interior, each with one weight per combination
+// of mirrored stencil cells (33 in 3D, 13 in 2D); passed to the kernel by value, so
+// that the weights are constant operands
+struct SymW {
+  double a[4][KFVM_MAX_CELLS];
 };
 
 // device-side scalars written by reductions

@@ -57,20 +57,36 @@ cudaError_t launch_dmma_peak(int blocks, int iters, double *out, cudaStream_t s)
 // of the reconstruction kernels, which read them)
 cudaError_t launch_bounds(int dim, int eq, const double *U, const Grid &g, double *bnd, cudaStream_t s);
 // stage front end: linear states + KXRCF indicator + limiter bound status,
-// KXRCF flags, WENO decision / heavy-list compaction, heavy cells
-// bnd: the limiter bounds of every cell from launch_bounds
-// (the FP64 form computes the limiter bounds itself and writes them to bnd).  umap
-// (recon_dmma_state_map of U; five variables, or GLM-MHD in 2D) stages the halo tiles by TMA;
-// null reads the state with plain global loads; a block whose wait gave up sets
-// sc->fault
+// KXRCF flags, WENO decision / heavy-list compaction, heavy cells.  The FP64
+// reconstruction computes the limiter bounds itself and writes them to bnd; a block
+// whose wait for its state tile gave up sets sc->fault.
+//
+// Two Gauss points per direction, not SR (recon_sym.cu): umap is recon_sym_state_map of U
+struct ReconSymArgs {
+  int wantInd;
+  double *const *F;
+  float *const *W;
+  double *src;
+  uint8_t *status;
+  double2 *lamvel;
+  double *bnd;
+  DevScalars *sc;
+};
+cudaError_t launch_recon_sym(int dim, int eq, const ReconSymArgs &a, const CUtensorMap &umap, const Grid &g,
+                             const SymW &w, cudaStream_t s);
+int recon_sym_state_map(CUtensorMap *map, const double *U, const Grid &g, int dim, int nv);
+// host: the parity weights of a stencil with two Gauss points; nonzero where the
+// weights of mirrored points are not mirror images
+int fill_sym_weights(const kfvm_stencil &st, bool interior, SymW &out);
+// Three Gauss points, and SR: umap (recon_dmma_state_map of U; five variables in 2D,
+// and SR) stages the halo tiles by TMA, null reads the state with plain global loads
 cudaError_t launch_recon(int dim, int eq, const double *U, const CUtensorMap *umap, const Grid &g,
                          const DevStencil *S, int wantInd, double *const *F, float *const *W, double *src,
                          uint8_t *status, double2 *lamvel, double *bnd, DevScalars *sc, cudaStream_t s);
 int recon_dmma_state_map(CUtensorMap *map, const double *U, const Grid &g, int dim, int nv);
 // the same outputs with the stencil sum on the tcgen05 tensor cores (3xTF32);
-// umap (recon_tc_state_map of U) stages the halo tiles by TMA, null loads them
-// with plain global loads; a block whose wait gave up sets sc->fault
-cudaError_t launch_recon_tc(int dim, int eq, const double *U, const CUtensorMap *umap, const Grid &g,
+// umap is recon_tc_state_map of U; a block whose wait gave up sets sc->fault
+cudaError_t launch_recon_tc(int dim, int eq, const double *U, const CUtensorMap &umap, const Grid &g,
                             const DevStencil *S, int wantInd, double *const *F, float *const *W, double *src,
                             uint8_t *status, double2 *lamvel, double *bnd, DevScalars *sc, cudaStream_t s);
 int recon_tc_state_map(CUtensorMap *map, const double *U, const Grid &g, int dim, int nv);

@@ -26,7 +26,7 @@ enum { DENS = 0, MOMX = 1, MOMY = 2, MOMZ = 3, ETOT = 4, MAGX = 5, MAGY = 6, MAG
 enum { EQ_HYDRO = 0, EQ_NS = 1, EQ_GLM = 2, EQ_SR = 3 };
 enum { RS_LLF = 0, RS_HLL = 1, RS_HLLC = 2 };
 
-// bound on the relative error of Eos::weno_approx.  For |log2 rho| <= 20 and
+// bound on the relative error of the indicator stored in 3D (Eos::weno_power32).  For |log2 rho| <= 20 and
 // gamma <= 3 the exponent -gamma lg2(rho) is off by at most gamma x 2 ulp(20)
 // = 1.2e-5 (lg2.approx) plus the FP32 roundings of gamma and of the product
 // (<= 5.5e-6), i.e. <= 1.8e-5 x ln 2 = 1.2e-5 relative after ex2; ex2.approx
@@ -39,9 +39,9 @@ constexpr double kWenoApproxEps = 2e-5;
 // 1e-14 of its scale.  The reconstruction of a uniform region leaves such
 // rounding-level differences between the two sides of a face.
 constexpr double kSameTol = 1e-14;
-// bound on the relative error of Eos::weno_round: one rounding to FP32 (2^-24)
-// plus a few FP64 ulps of the pressure, the power and the quotient
-constexpr double kWenoRoundEps = 6.0e-8;
+// bound on the relative error of the indicator stored in 2D: one rounding to FP32
+// (2^-24 = 5.97e-8) and the 1e-9 of Eos::weno_power64 (SR stores the rounded density)
+constexpr double kWenoRoundEps = 6.2e-8;
 
 // Reciprocal by Newton-Raphson refinement (Flynn 1970; Markstein 1990) of the
 // hardware's approximate FP64 reciprocal (PTX rcp.approx.ftz.f64): each step
@@ -117,39 +117,71 @@ struct Eos {
     if constexpr (EQ == EQ_SR) return U[DENS];
     else return pres(g, U) / pow(U[DENS], g);
   }
-  // The same indicator with the power taken in FP32 by the hardware lg2 / ex2
-  // approximations (the pressure stays FP64): relative error below
-  // kWenoApproxEps for densities in [2^-20, 2^20] and 1 < gamma <= 3.  Outside
-  // that range, or for a non-finite pressure, it returns NaN, which tells the
-  // reader to recompute the exact value.
-  __device__ __forceinline__ static float weno_approx(double g, const double *U) {
-    return weno_approx_rp(g, U[DENS], pres(g, U));
-  }
-  // the same from density and pressure
-  __device__ __forceinline__ static float weno_approx_rp(double g, double rho, double p) {
-    if (!(rho >= 9.5367431640625e-07 && rho <= 1048576.0) || !(g <= 3.0) || !isfinite(p))
-      return __int_as_float(0x7fc00000);
+  // The indicator as the reconstruction stores it, in FP32, in two steps: the power
+  // rho^-gamma, then its product with the pressure.  Both steps give NaN where their
+  // error bound does not hold, which tells the reader to recompute the exact value.
+  //
+  // In 3D (24 face points) the power comes from the hardware lg2 / ex2 approximations:
+  // relative error below kWenoApproxEps for densities in [2^-20, 2^20) and gamma <= 3.
+  __device__ __forceinline__ static float weno_power32(double g, double rho) {
+    // the density's exponent and sign in one integer comparison
+    const unsigned hi = (unsigned)__double2hiint(rho) - 0x3eb00000u;
+    if (hi >= 0x02800000u || !(g <= 3.0)) return __int_as_float(0x7fc00000);
     float l2, r;
-    asm("lg2.approx.f32 %0, %1;" : "=f"(l2) : "f"((float)rho));
-    asm("ex2.approx.f32 %0, %1;" : "=f"(r) : "f"(-(float)g * l2));
-    const float w = (float)p * r;
-    // an FP32 underflow (or overflow) of the product voids the bound
-    return fabsf(w) >= 1.17549435e-38f ? w : __int_as_float(0x7fc00000);
+    asm("lg2.approx.ftz.f32 %0, %1;" : "=f"(l2) : "f"((float)rho));  // normal in, normal out
+    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(-(float)g * l2));
+    return r;
   }
-  // The indicator computed in FP64 as the reference does and rounded once to FP32
-  // (relative error below kWenoRoundEps), or NaN where FP32 cannot hold it
-  __device__ __forceinline__ static float weno_round_rp(double g, double rho, double p) {
-    const float w = __double2float_rn(p / pow(rho, g));
+  // In 2D (8 face points; fine grids put smooth cells' jumps close to the threshold)
+  // it is an FP64 value good to 1e-9.  With rho = 2^e m, m in [1/sqrt 2, sqrt 2), and
+  // z = (m - 1) / (m + 1), log2 m = 2 / ln 2 (z + z^3 / 3 + z^5 / 5 + ...): |z| < 0.1716,
+  // so the terms from z^13 on are below 3e-11.  Then 2^f for |f| <= 1/2 is the
+  // exponential series to the 8th power (the rest is below 3e-10).  About 30
+  // operations, where the library's correctly rounded-to-1-ulp power takes several
+  // times as many for digits that the rounding to FP32 drops.
+  __device__ __forceinline__ static double weno_power64(double g, double rho) {
+    const double nan = __longlong_as_double(0x7ff8000000000000ll);
+    if (!(rho >= 1e-290 && rho <= 1e290)) return nan;
+    int hi = __double2hiint(rho), e = (hi >> 20) - 1023;
+    double m = __hiloint2double((hi & 0xfffff) | 0x3ff00000, __double2loint(rho));
+    if (m > 1.4142135623730951) {
+      m *= 0.5;
+      e++;
+    }
+    const double z = (m - 1.0) * rcp_nr(m + 1.0), z2 = z * z;
+    constexpr double k = 2.8853900817779268;  // 2 / ln 2
+    double l = fma(z2, k / 11.0, k / 9.0);
+    l = fma(z2, l, k / 7.0);
+    l = fma(z2, l, k / 5.0);
+    l = fma(z2, l, k / 3.0);
+    l = fma(z2, l, k);
+    const double t = -g * fma(z, l, (double)e);
+    if (!(fabs(t) < 1000.0)) return nan;
+    const double n = rint(t), x = (t - n) * 0.6931471805599453;
+    double r = fma(x, 1.0 / 40320.0, 1.0 / 5040.0);
+    r = fma(x, r, 1.0 / 720.0);
+    r = fma(x, r, 1.0 / 120.0);
+    r = fma(x, r, 1.0 / 24.0);
+    r = fma(x, r, 1.0 / 6.0);
+    r = fma(x, r, 0.5);
+    r = fma(x, r, 1.0);
+    r = fma(x, r, 1.0);
+    return __hiloint2double(__double2hiint(r) + ((int)n << 20), __double2loint(r));
+  }
+  template <int DIM>
+  __device__ __forceinline__ static auto weno_power(double g, double rho) {
+    if constexpr (DIM == 2) return weno_power64(g, rho);
+    else return weno_power32(g, rho);
+  }
+  // an FP32 underflow or overflow voids the bounds
+  template <int DIM, class P>
+  __device__ __forceinline__ static float weno_from_power(double p, P power) {
+    const float w = DIM == 2 ? __double2float_rn(p * (double)power) : (float)p * (float)power;
     return fabsf(w) >= 1.17549435e-38f && fabsf(w) <= 3.0e38f ? w : __int_as_float(0x7fc00000);
   }
-  // the FP32 form the reconstruction stores: in 2D (8 face points per cell, where
-  // the power is cheap next to the rest and fine grids put smooth cells' jumps
-  // close to the threshold) the rounded FP64 value; in 3D (24 points) the
-  // hardware approximation
   template <int DIM>
   __device__ __forceinline__ static float weno_store(double g, double rho, double p) {
-    if constexpr (DIM == 2) return weno_round_rp(g, rho, p);
-    else return weno_approx_rp(g, rho, p);
+    return weno_from_power<DIM>(p, weno_power<DIM>(g, rho));
   }
   __device__ __forceinline__ static double positivity(const double *U) {
     if constexpr (EQ == EQ_SR) return sr::positivity(U);

@@ -1,7 +1,7 @@
 // recon_tc.cu -- the linear reconstruction contraction on the tcgen05 tensor cores
 // (the FP32 form: 3xTF32 products, FP32 accumulation in tensor memory).
 //
-// Same outputs as recon_kernel (KernelLinearRecon_K, src/stencil/Stencil_K.H:56-119
+// Same outputs as recon_sym.cu's kernels (KernelLinearRecon_K, src/stencil/Stencil_K.H:56-119
 // of the reference, plus the KXRCF indicator and the positivity pre-check), with
 // the sum over stencil cells done as one MMA tile per block of 128 cells:
 //
@@ -89,217 +89,13 @@ struct TcShape {
 };
 
 // ---------------------------------------------------------------------------
-template <int DIM, int EQ>
-__global__ void __launch_bounds__(kTcThreads, 2)
-    recon_tc_kernel(const double *__restrict__ U, Grid g, const DevStencil *__restrict__ S, int wantInd,
-                    double *__restrict__ F0, double *__restrict__ F1, double *__restrict__ F2,
-                    float *__restrict__ W0, float *__restrict__ W1, float *__restrict__ W2,
-                    double *__restrict__ src, uint8_t *__restrict__ status, double2 *__restrict__ lamvel,
-                    double *__restrict__ bnd, DevScalars *__restrict__ sc) {
-  using T = Cfg<DIM, EQ>;
-  using Sh = TcShape<DIM, EQ>;
-  constexpr int NV = T::NV;
-  extern __shared__ __align__(128) uint8_t smem[];
-  double(*sBd)[128] = reinterpret_cast<double(*)[128]>(smem + Sh::OFF_BD);
-  unsigned long long *sLam = reinterpret_cast<unsigned long long *>(smem + Sh::OFF_RED);
-  unsigned long long *sVel = sLam + 128;
-  int *sIn = reinterpret_cast<int *>(smem + Sh::OFF_RED + 2 * 128 * 8);
-  uint64_t *bar = reinterpret_cast<uint64_t *>(smem + Sh::OFF_BAR);
-  uint32_t *tslot = reinterpret_cast<uint32_t *>(smem + Sh::OFF_BAR + 8);
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int quarter = warp & 3, part = warp >> 2;
-  const int row = quarter * 32 + lane;     // tile row = TMEM lane = cell (lane, quarter) of the block
-  const int tid = threadIdx.x;
-  const int64_t i = blockIdx.x * (int64_t)kBlockX + lane;
-  const int64_t j = blockIdx.y * (int64_t)kBlockY + quarter;
-  const int64_t k = blockIdx.z;
-  const bool live = i < g.nx && j < g.ny;
-  const uint32_t barA = smem_u32(bar);
-
-  if (warp == 0) {
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tslot)),
-                 "r"((uint32_t)Sh::COLS)
-                 : "memory");
-    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
-  }
-  if (tid == 0) {
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(barA) : "memory");
-    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-  }
-  // B operand (split weights, already in core-matrix order) and the limiter tile
-  {
-    const float4 *bh = reinterpret_cast<const float4 *>(S->tcw[0]);
-    const float4 *bl = reinterpret_cast<const float4 *>(S->tcw[1]);
-    float4 *dh = reinterpret_cast<float4 *>(smem + Sh::OFF_B);
-    float4 *dl = reinterpret_cast<float4 *>(smem + Sh::OFF_B + Sh::B_PART);
-    for (int t = tid; t < Sh::B_PART / 16; t += kTcThreads) {
-      dh[t] = bh[t];
-      dl[t] = bl[t];
-    }
-  }
-  if (part == 0) {
-    sIn[row] = 1;
-    sLam[row] = 0ull;
-    sVel[row] = 0ull;
-    if (live) {
-      // limiter bounds of the cell (bounds_kernel)
-      const int64_t c = (k * g.ny + j) * g.nx + i;
-      sBd[0][row] = bnd[c];
-      sBd[1][row] = bnd[g.n + c];
-      sBd[2][row] = bnd[2 * g.n + c];
-    }
-  }
-  asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-  __syncthreads();
-  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-  const uint32_t tmem = *tslot;
-
-  const double *Uc = U + pidx(g, live ? i : 0, live ? j : 0, k);
-  const uint32_t aHi = smem_u32(smem), aLo = aHi + Sh::A_PART;
-  const uint32_t bHi = smem_u32(smem + Sh::OFF_B), bLo = bHi + Sh::B_PART;
-  constexpr uint32_t idesc = tf32_idesc<Sh::NP>();
-
-  bool ok = true;
-#pragma unroll 1
-  for (int v = 0; v < NV; v++) {
-    if (v > 0) ok = mbar_wait(barA, (uint32_t)(v - 1) & 1u);
-    if (!__syncthreads_and(ok)) break;
-    // this thread's share of the A row for variable v: chunks part, part + 2, ...
-    const double *Uv = Uc + v * g.pvol;
-    const double ucv = live ? Uv[0] : 0.0;
-#pragma unroll
-    for (int ch = part; ch < Sh::NCH; ch += kTcParts) {
-      uint32_t hi[4], lo[4];
-#pragma unroll
-      for (int t = 0; t < 4; t++) {
-        const int c = ch * 4 + t;
-        float d = 0.0f;
-        if (c < T::C && live) d = (float)(__ldg(Uv + g.loff[c]) - ucv);
-        hi[t] = to_tf32(d);
-        lo[t] = to_tf32(d - __uint_as_float(hi[t]));
-      }
-      st_shared_v4(aHi + ch * Sh::A_CH + row * 16, hi);
-      st_shared_v4(aLo + ch * Sh::A_CH + row * 16, lo);
-    }
-    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-    __syncthreads();
-    if (tid == 0) {
-      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-      const uint32_t d = tmem + (uint32_t)(v * Sh::NP);
-#pragma unroll
-      for (int s = 0; s < Sh::NKS; s++) {
-        const uint64_t ah = umma_desc(aHi + 2 * s * Sh::A_CH, Sh::A_CH, 128);
-        const uint64_t al = umma_desc(aLo + 2 * s * Sh::A_CH, Sh::A_CH, 128);
-        const uint64_t bh = umma_desc(bHi + 2 * s * Sh::B_CH, Sh::B_CH, 128);
-        const uint64_t bl = umma_desc(bLo + 2 * s * Sh::B_CH, Sh::B_CH, 128);
-        mma_tf32(d, al, bh, idesc, s > 0);
-        mma_tf32(d, ah, bl, idesc, 1);
-        mma_tf32(d, ah, bh, idesc, 1);
-      }
-      mma_commit(barA);
-    }
-  }
-  if (ok) ok = mbar_wait(barA, (uint32_t)(NV - 1) & 1u);
-  if (__syncthreads_and(ok)) {
-    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    PosBounds bd;
-    bd.minDens = sBd[0][row];
-    bd.maxDens = sBd[1][row];
-    bd.minEint = sBd[2][row];
-    double uc[NV];
-#pragma unroll
-    for (int v = 0; v < NV; v++) uc[v] = live ? Uc[v * g.pvol] : 0.0;
-    const uint32_t lanes = (uint32_t)(quarter * 32) << 16;
-    const int64_t c = (k * g.ny + j) * g.nx + i;
-    bool inside = true;
-    double lam = 0.0, vel = 0.0;
-    // the rows of each part are known at compile time (face, direction, point)
-    auto epilogue = [&](auto partTag) {
-      constexpr int PART = decltype(partTag)::value;
-      constexpr int R0 = PART * Sh::RPP;
-#pragma unroll
-      for (int rp = 0; rp < Sh::RPP; rp += 2) {
-        float a0[NV], a1[NV];
-        tmem_ld2_n<NV>(tmem + lanes + (uint32_t)(R0 + rp), (uint32_t)Sh::NP, a0, a1);
-        if (live) {
-#pragma unroll
-          for (int e = 0; e < 2; e++) {
-            const int rw = R0 + rp + e;
-            if (rw < Sh::NR) {
-              double st[NV];
-#pragma unroll
-              for (int v = 0; v < NV; v++) st[v] = uc[v] + (double)(e ? a1[v] : a0[v]);
-              // pos_inside, with the internal energy kept for the indicator's pressure
-              // Euler / Navier-Stokes: the certified internal energy (no IEEE division)
-              double ei;
-              if constexpr (EQ == EQ_GLM) ei = Eos<EQ>::eint(st);
-              else ei = Eos<EQ>::eint_vs(st, bd.minEint);
-              inside = inside && st[DENS] > bd.minDens && st[DENS] < bd.maxDens && ei > bd.minEint;
-              if (rw < T::NF * T::NQF) {
-                const int f = rw / T::NQF, q = rw % T::NQF, d = f >> 1;
-                double *Fd = d == 0 ? F0 : (d == 1 ? F1 : F2);
-                const int64_t a = face_slot_addr(g, f, i, j, k, q, 0, T::NQF, NV);
-                const int64_t nf = g.nface[d];
-#pragma unroll
-                for (int v = 0; v < NV; v++) Fd[a + v * nf] = st[v];
-                if (wantInd)
-                  (d == 0 ? W0 : (d == 1 ? W1 : W2))[face_slot_addr(g, f, i, j, k, q, 0, T::NQF, 1)] =
-                      Eos<EQ>::template weno_store<DIM>(g.gamma, st[DENS], (g.gamma - 1.0) * ei);
-                if constexpr (T::SRC) {
-                  // SpeedEstimate_K<MHD_GLM> (MHD_GLM_K.H:213-310): x components on every face
-                  const double vv = fabs(st[MOMX] / st[DENS]);
-                  const double l = Eos<EQ>::fastMagSonic(g.gamma, st, st[MAGX]) + vv;
-                  vel = vv > vel ? vv : vel;
-                  lam = l > lam ? l : lam;
-                }
-              } else if constexpr (T::SRC) {
-                const int q = rw - T::NF * T::NQF;
-#pragma unroll
-                for (int v = 0; v < NV; v++) src[(q * NV + v) * g.n + c] = st[v];
-              }
-            }
-          }
-        }
-      }
-    };
-    static_assert(kTcParts == 2, "epilogue specialised for two parts");
-    if (part == 0) epilogue(std::integral_constant<int, 0>{});
-    else epilogue(std::integral_constant<int, 1>{});
-    // combine the two parts of each cell
-    if (live && !inside) atomicAnd(&sIn[row], 0);
-    if constexpr (T::SRC) {
-      if (live) {
-        if (lam >= 0.0) atomicMax(&sLam[row], (unsigned long long)__double_as_longlong(lam));
-        if (vel >= 0.0) atomicMax(&sVel[row], (unsigned long long)__double_as_longlong(vel));
-      }
-    }
-    __syncthreads();
-    if (live && part == 0) {
-      if constexpr (T::SRC)
-        lamvel[c] = make_double2(__longlong_as_double((long long)sLam[row]), __longlong_as_double((long long)sVel[row]));
-      status[c] = sIn[row] ? 1 : 0;
-    }
-  } else if (tid == 0) {
-    atomicExch(&sc->fault, 1u);
-  }
-  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-  __syncthreads();
-  if (warp == 0)
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"((uint32_t)Sh::COLS)
-                 : "memory");
-}
-
-// ---------------------------------------------------------------------------
-// The same contraction with the halo tile staged by TMA.  Per variable v one 4D
+// The halo tile is staged by TMA.  Per variable v one 4D
 // tensor load (x, y, z, v of the padded state; box 36 x 8 x 5 in 3D, 36 x 8 x 1 in
 // 2D) brings the block's stencil footprint into shared memory; the A rows are
-// built from it (the same FP64 differences as above, so the products are the
-// same bits), and the load of variable v + 2 is issued as soon as the build
+// built from it, and the load of variable v + 2 is issued as soon as the build
 // of v - 1 has read its buffer (three buffers: loads run two variables ahead of
 // the build).  The cell averages of the block are kept in shared memory for the
-// FP64 epilogue; the limiter bounds come from bounds_kernel.  Used when the padded
-// row pitch is even (TMA strides are multiples of 16 bytes).
+// FP64 epilogue; the limiter bounds come from bounds_kernel.
 template <int DIM>
 struct HaloTile {
   static constexpr int R = 2;
@@ -584,32 +380,23 @@ cudaError_t launch_wait_probe(uint64_t limit_ns, unsigned long long *out, cudaSt
 }
 
 template <int DIM, int EQ>
-static cudaError_t recon_tc_launch(const double *U, const CUtensorMap *umap, const Grid &g, const DevStencil *S,
+static cudaError_t recon_tc_launch(const double *U, const CUtensorMap &umap, const Grid &g, const DevStencil *S,
                                    int wantInd, double *const *F, float *const *W, double *src, uint8_t *status,
                                    double2 *lamvel, double *bnd, DevScalars *sc, cudaStream_t s) {
-  using Sh = TcShape<DIM, EQ>;
   using L = TcTmaShape<DIM, EQ>;
   const dim3 grid((unsigned)((g.nx + kBlockX - 1) / kBlockX), (unsigned)((g.ny + kBlockY - 1) / kBlockY),
                   (unsigned)g.nz);
-  if (umap) {
-    // the attribute is per function and process-wide: set once (a function-local
-    // static is initialised once, also when several host threads drive solvers)
-    static const cudaError_t attrT =
-        cudaFuncSetAttribute(recon_tc_tma_kernel<DIM, EQ>, cudaFuncAttributeMaxDynamicSharedMemorySize, L::SMEM);
-    if (attrT != cudaSuccess) return attrT;
-    recon_tc_tma_kernel<DIM, EQ><<<grid, kTcThreads, L::SMEM, s>>>(
-        *umap, U, g, S, wantInd, F[0], F[1], F[2], W[0], W[1], W[2], src, status, lamvel, bnd, sc);
-    return cudaGetLastError();
-  }
-  static const cudaError_t attr =
-      cudaFuncSetAttribute(recon_tc_kernel<DIM, EQ>, cudaFuncAttributeMaxDynamicSharedMemorySize, Sh::SMEM);
-  if (attr != cudaSuccess) return attr;
-  recon_tc_kernel<DIM, EQ><<<grid, kTcThreads, Sh::SMEM, s>>>(
-      U, g, S, wantInd, F[0], F[1], F[2], W[0], W[1], W[2], src, status, lamvel, bnd, sc);
+  // the attribute is per function and process-wide: set once (a function-local
+  // static is initialised once, also when several host threads drive solvers)
+  static const cudaError_t attrT =
+      cudaFuncSetAttribute(recon_tc_tma_kernel<DIM, EQ>, cudaFuncAttributeMaxDynamicSharedMemorySize, L::SMEM);
+  if (attrT != cudaSuccess) return attrT;
+  recon_tc_tma_kernel<DIM, EQ><<<grid, kTcThreads, L::SMEM, s>>>(
+      umap, U, g, S, wantInd, F[0], F[1], F[2], W[0], W[1], W[2], src, status, lamvel, bnd, sc);
   return cudaGetLastError();
 }
 
-cudaError_t launch_recon_tc(int dim, int eq, const double *U, const CUtensorMap *umap, const Grid &g,
+cudaError_t launch_recon_tc(int dim, int eq, const double *U, const CUtensorMap &umap, const Grid &g,
                             const DevStencil *S, int wantInd, double *const *F, float *const *W, double *src,
                             uint8_t *status, double2 *lamvel, double *bnd, DevScalars *sc, cudaStream_t s) {
   if (dim == 2) {
@@ -622,10 +409,8 @@ cudaError_t launch_recon_tc(int dim, int eq, const double *U, const CUtensorMap 
   return recon_tc_launch<3, EQ_HYDRO>(U, umap, g, S, wantInd, F, W, src, status, lamvel, bnd, sc, s);
 }
 
-// 4D map (x, y, z, variable) of a padded state for the halo-tile loads, or a
-// nonzero return where TMA cannot address it (odd row pitch)
+// 4D map (x, y, z, variable) of a padded state for the halo-tile loads
 int recon_tc_state_map(CUtensorMap *map, const double *U, const Grid &g, int dim, int nv) {
-  if (g.px % 2 != 0) return 1;
   const uint64_t planes = (uint64_t)(g.pvol / (g.px * g.py));
   const uint64_t dims[4] = {(uint64_t)g.px, (uint64_t)g.py, planes, (uint64_t)nv};
   const uint64_t strides[3] = {(uint64_t)g.px * 8, (uint64_t)(g.px * g.py) * 8, (uint64_t)g.pvol * 8};
