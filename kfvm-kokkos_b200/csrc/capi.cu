@@ -614,7 +614,7 @@ int eval_front(kfvm_solver *s, int b) {
       CK(cudaStreamSynchronize(st));
     }
   }
-  if ((e = run(s, KFVM_KCLASS_RIEMANN, dim,
+  if ((e = run(s, KFVM_KCLASS_RIEMANN, 1,
                [&] { return launch_riemann(dim, eq, s->F, s->G, s->g, s->sc, s->sameOn, st); })) !=
       cudaSuccess)
     return set_err_cuda(e, "riemann");

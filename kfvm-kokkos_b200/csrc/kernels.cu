@@ -1520,70 +1520,96 @@ __global__ void __launch_bounds__(HeavyShape<DIM, EQ, NQ>::CELLS * Eos<EQ>::NV, 
 }
 
 // ---------------------------------------------------------------------------
-// Riemann fluxes of direction D: one thread per face point (block = 32 faces x NQF
-// points, points along threadIdx.y), so each thread keeps only one solve live and
-// more warps hide the FP64 latency.  The quadrature-weighted sum over a face's
-// points goes through shared memory in point order, and the max wave speed
-// through a warp maximum and an atomic only from warps that raise it.
-// SAME: faces whose two states agree to kSameTol take the consistent flux F(u)
-// without the wave fan (Eos::solve_same); one block in
-// kSameSample counts such faces so that the host can fall back to the plain
-// variant where few faces qualify (its slow path spills more registers).
+// Riemann fluxes: one thread per face point (block = 32 faces x NQF points, points along
+// threadIdx.y; two such rows of faces in 2D), so each thread keeps only one solve live
+// and more warps hide the FP64 latency.  One launch takes all directions (blockIdx.z).
+// The quadrature-weighted sum over a face's points goes through shared memory in point
+// order, the variables shared among the face's warps; the max wave speed through a warp
+// maximum of the bit patterns (two integer reductions) and an atomic only from warps
+// that raise it.
+// SAME: faces whose two states agree take the consistent flux F(u) without the wave
+// fan (Eos::solve_same); one block in kSameSample counts such faces so that the host
+// can fall back to the plain variant where few faces qualify.
+// Bound by the issue rate (608 instructions a point, 249 of them FP64, where it had 824
+// and 319).  Per evaluation: Navier-Stokes 160^3 1.42 -> 1.10 ms, Euler 1024^2 0.135 ->
+// 0.103, GLM-MHD 1024^2 0.26 -> 0.148 and 96^3 0.58 -> 0.35, SR 512^2 0.32 -> 0.25; Euler
+// 32^2, where the launch counts, 13.8 -> 8.6 us.
 constexpr int kSameSample = 1024;
 
+// the largest value over the warp, as bits, of non-negative doubles (NaN counts as 0)
+__device__ __forceinline__ unsigned long long warp_max_bits(double v) {
+  const unsigned long long b = v >= 0.0 ? (unsigned long long)__double_as_longlong(v) : 0ull;
+  const unsigned hi = (unsigned)(b >> 32), mh = __reduce_max_sync(0xffffffffu, hi);
+  const unsigned ml = __reduce_max_sync(0xffffffffu, hi == mh ? (unsigned)b : 0u);
+  return (unsigned long long)mh << 32 | ml;
+}
+
+template <int DIM, int EQ, int NQ>
+struct RiemannShape {
+  static constexpr int NQF = Cfg<DIM, EQ, NQ>::NQF;
+  static constexpr int ROWS = DIM == 2 ? 2 : 1;   // rows of 32 faces per block
+  static constexpr int THREADS = 32 * NQF * ROWS;
+  static constexpr int RESIDENT =
+      EQ == EQ_GLM ? 1 : (EQ == EQ_SR ? 4 : (DIM == 2 ? (NQ == 3 ? 5 : 8) : (NQ == 3 ? 3 : 8)));
+};
+
 template <int DIM, int EQ, int D, int NQ, bool SAME>
-__global__ void __launch_bounds__(32 * Cfg<DIM, EQ, NQ>::NQF,
-                                  EQ == EQ_GLM ? 1
-                                               : (EQ == EQ_SR ? (DIM == 2 ? 8 : 4)
-                                                              : (DIM == 2 ? 16 : (NQ == 3 ? 7 : 8))))
-    riemann_kernel(const double *__restrict__ F, double *__restrict__ G, Grid g,
-                   DevScalars *__restrict__ sc) {
+__device__ __forceinline__ void riemann_dir(const double *__restrict__ F, double *__restrict__ G, const Grid &g,
+                                            uint64_t fdiv, DevScalars *__restrict__ sc,
+                                            double (*part)[Cfg<DIM, EQ, NQ>::NQF][Eos<EQ>::NV][32], unsigned *cnt) {
   using T = Cfg<DIM, EQ, NQ>;
   using E = Eos<EQ>;
+  using R = RiemannShape<DIM, EQ, NQ>;
   constexpr int NV = T::NV, NQF = T::NQF;
-  __shared__ double part[NQF][NV][32];
-  const int64_t fx = g.fdim[D][0], fy = g.fdim[D][1], nf = g.nface[D];
-  // the face within its (x, y) plane, split with 32-bit arithmetic (a plane holds
-  // far fewer than 2^32 faces)
-  const unsigned flat = blockIdx.x * 32u + threadIdx.x, ux = (unsigned)fx;
-  const unsigned jj = flat / ux;
-  const int64_t i = (int64_t)(flat - jj * ux), j = jj;
-  const int64_t k = blockIdx.z;
-  const int q = threadIdx.y;
+  const int64_t fx = g.fdim[D][0], nf = g.nface[D];
+  const int q = threadIdx.y % NQF, row = threadIdx.y / NQF;
+  // the face within its (x, y) plane, split by a multiplication with 2^64 / fx (exact
+  // for 32-bit indices; a plane holds far fewer than 2^32 faces)
+  const unsigned flat = (blockIdx.x * R::ROWS + row) * 32u + threadIdx.x;
+  const unsigned j = (unsigned)__umul64hi(flat, fdiv), i = flat - j * (unsigned)fx;
+  const unsigned k = blockIdx.y;
   double vmax = 0.0;
-  const bool live = j < fy;
+  const bool live = j < (unsigned)g.fdim[D][1];
   bool same = false;
+  const int64_t fidx = (int64_t)k * (fx * g.fdim[D][1]) + flat;
   if (live) {
-    const int64_t fidx = (k * fy + j) * fx + i;
-    const int64_t m = D == 0 ? i : (D == 1 ? j : k);
-    const int64_t nd = D == 0 ? g.nx : (D == 1 ? g.ny : g.nz);
+    const unsigned m = D == 0 ? i : (D == 1 ? j : k);
+    const unsigned nd = (unsigned)(D == 0 ? g.nx : (D == 1 ? g.ny : g.nz));
     // face BCs (setFaceBCs): boundary faces take the missing slot from the
     // periodic partner face, or copy the interior slot at an outflow boundary
-    int64_t f0 = fidx, f1 = fidx;
-    int s0 = 0, s1 = 1;
-    const int64_t stride = D == 0 ? 1 : (D == 1 ? fx : fx * fy);
-    // (an exchange or user face holds the outer state in its own outer slot)
-    if (m == 0) {
-      if (g.bc[2 * D] == KFVM_BC_PERIODIC) f0 = fidx + nd * stride;
-      else if (!outer_in_face(g.bc[2 * D])) s0 = 1;
-    } else if (m == nd) {
-      if (g.bc[2 * D + 1] == KFVM_BC_PERIODIC) f1 = fidx - nd * stride;
-      else if (!outer_in_face(g.bc[2 * D + 1])) s1 = 0;
+    const double *pL = F + (int64_t)q * NV * nf + fidx, *pR = pL + (int64_t)NQF * NV * nf;
+    unsigned flipL = 0u, flipR = 0u;
+    if (m == 0 || m == nd) {
+      const int64_t stride = D == 0 ? 1 : (D == 1 ? fx : fx * g.fdim[D][1]);
+      const int bc = g.bc[2 * D + (m != 0)];
+      // (an exchange or user face holds the outer state in its own outer slot; a wall
+      // face, reflecting or no-slip, mirrors the inner state with sign flips)
+      if (m == 0) {
+        if (bc == KFVM_BC_PERIODIC) pL += (int64_t)nd * stride;
+        else if (!outer_in_face(bc)) {
+          pL = pR;
+          flipL = g.bflip[2 * D];
+        }
+      } else {
+        if (bc == KFVM_BC_PERIODIC) pR -= (int64_t)nd * stride;
+        else if (!outer_in_face(bc)) {
+          pR = pL;
+          flipR = g.bflip[2 * D + 1];
+        }
+      }
     }
     const double ch = EQ == EQ_GLM ? __longlong_as_double((long long)sc->glm_lam_bits) -
                                          __longlong_as_double((long long)sc->glm_vel_bits)
                                    : 0.0;
     double uL[NV], uR[NV], Fq[NV];
-    const double *pL = F + (int64_t)(s0 * NQF + q) * NV * nf + f0;
-    const double *pR = F + (int64_t)(s1 * NQF + q) * NV * nf + f1;
 #pragma unroll
     for (int v = 0; v < NV; v++) {
-      uL[v] = __ldg(pL + v * nf);
-      uR[v] = __ldg(pR + v * nf);
+      uL[v] = __ldg(pL);
+      uR[v] = __ldg(pR);
+      pL += nf;
+      pR += nf;
     }
-    if (s0 == 1 || s1 == 0) {
-      // a wall face (reflecting / no-slip) mirrors the inner state with sign flips
-      const unsigned flipL = s0 == 1 ? g.bflip[2 * D] : 0u, flipR = s1 == 0 ? g.bflip[2 * D + 1] : 0u;
+    if (flipL | flipR) {
 #pragma unroll
       for (int v = 0; v < NV; v++) {
         if ((flipL >> v) & 1u) uL[v] = -uL[v];
@@ -1591,8 +1617,8 @@ __global__ void __launch_bounds__(32 * Cfg<DIM, EQ, NQ>::NQF,
       }
     }
     if constexpr (SAME) {
-      // a face inside a uniform region needs no wave fan (kSameTol)
-      same = E::same_state(uL, uR);
+      // a face inside a uniform region needs no wave fan
+      same = E::template same_state<NQ == 2 && EQ != EQ_SR>(uL, uR);
       if (same) vmax = E::solve_same(g.gamma, ch, D, uL, Fq);
       else vmax = E::solve(g.rs, g.gamma, ch, D, uL, uR, Fq);
     } else {
@@ -1601,11 +1627,10 @@ __global__ void __launch_bounds__(32 * Cfg<DIM, EQ, NQ>::NQF,
     // Gauss weight of point q (3D: the product of the two transverse weights)
     const double wq = DIM == 2 ? gl_wt<NQ>(q) : gl_wt<NQ>(q / NQ) * gl_wt<NQ>(q % NQ);
 #pragma unroll
-    for (int v = 0; v < NV; v++) part[q][v][threadIdx.x] = wq * Fq[v];
+    for (int v = 0; v < NV; v++) part[row][q][v][threadIdx.x] = wq * Fq[v];
   }
-  __shared__ unsigned cnt[2];
-  const bool sampled = SAME && (blockIdx.x + 11u * blockIdx.z) % kSameSample == 0;
-  if (sampled && threadIdx.x == 0 && q == 0) cnt[0] = cnt[1] = 0u;
+  const bool sampled = SAME && (blockIdx.x + 11u * k) % kSameSample == 0;
+  if (sampled && threadIdx.x == 0 && threadIdx.y == 0) cnt[0] = cnt[1] = 0u;
   __syncthreads();
   if (sampled) {
     const unsigned bs = __ballot_sync(0xffffffffu, same), bl = __ballot_sync(0xffffffffu, live);
@@ -1614,25 +1639,48 @@ __global__ void __launch_bounds__(32 * Cfg<DIM, EQ, NQ>::NQF,
       atomicAdd(&cnt[1], (unsigned)__popc(bl));
     }
   }
-  if (live && q == 0) {
-    const int64_t fidx = (k * fy + j) * fx + i;
+  if (live) {
 #pragma unroll
-    for (int v = 0; v < NV; v++) {
-      double acc = 0.0;
+    for (int v0 = 0; v0 < NV; v0 += NQF) {
+      const int v = v0 + q;
+      if (v < NV) {
+        double acc = 0.0;
 #pragma unroll
-      for (int p = 0; p < NQF; p++) acc += part[p][v][threadIdx.x];
-      G[(int64_t)v * nf + fidx] = acc;
+        for (int p = 0; p < NQF; p++) acc += part[row][p][v][threadIdx.x];
+        G[(int64_t)v * nf + fidx] = acc;
+      }
     }
   }
-  vmax = warp_max(vmax);
-  if (threadIdx.x == 0) atomic_max_pos(&sc->maxvel_bits, vmax);
+  const unsigned long long top = warp_max_bits(vmax);
+  if (threadIdx.x == 0 && top > *(volatile const unsigned long long *)&sc->maxvel_bits)
+    atomicMax(&sc->maxvel_bits, top);
   if (sampled) {
     __syncthreads();
-    if (threadIdx.x == 0 && q == 0) {
+    if (threadIdx.x == 0 && threadIdx.y == 0) {
       atomicAdd(&sc->nsame, (unsigned long long)cnt[0]);
       atomicAdd(&sc->nsamp, (unsigned long long)cnt[1]);
     }
   }
+}
+
+struct RiemannArgs {
+  const double *F[3];
+  double *G[3];
+  uint64_t fdiv[3];     // 2^64 / (faces per row), rounded up
+  unsigned blocks[3];   // blocks per plane
+};
+
+template <int DIM, int EQ, int NQ, bool SAME>
+__global__ void __launch_bounds__(RiemannShape<DIM, EQ, NQ>::THREADS, RiemannShape<DIM, EQ, NQ>::RESIDENT)
+    riemann_kernel(const __grid_constant__ RiemannArgs a, const __grid_constant__ Grid g, DevScalars *__restrict__ sc) {
+  using R = RiemannShape<DIM, EQ, NQ>;
+  __shared__ double part[R::ROWS][R::NQF][Eos<EQ>::NV][32];
+  __shared__ unsigned cnt[2];
+  const int d = blockIdx.z;
+  if (blockIdx.x >= a.blocks[d] || blockIdx.y >= (unsigned)g.fdim[d][2]) return;
+  if (d == 0) riemann_dir<DIM, EQ, 0, NQ, SAME>(a.F[0], a.G[0], g, a.fdiv[0], sc, part, cnt);
+  else if (d == 1) riemann_dir<DIM, EQ, 1, NQ, SAME>(a.F[1], a.G[1], g, a.fdiv[1], sc, part, cnt);
+  else riemann_dir<DIM, EQ, DIM == 3 ? 2 : 1, NQ, SAME>(a.F[DIM - 1], a.G[DIM - 1], g, a.fdiv[DIM - 1], sc, part, cnt);
 }
 
 // ---------------------------------------------------------------------------
@@ -2175,25 +2223,23 @@ struct Launch {
         U, g, S, theta, F[0], F[1], F[2], src, heavy, bnd, sc, jd);
     return cudaGetLastError();
   }
-  template <bool SAME>
-  static void riemann_dirs(double *const *F, double *const *G, const Grid &g, DevScalars *sc, cudaStream_t s) {
-#pragma unroll 1
-    for (int d = 0; d < DIM; d++) {
-      // 32 consecutive faces of an (x, y) face plane per block (rows of the x faces
-      // hold nx + 1 faces, which would leave a nearly empty block per row), NQF
-      // points along threadIdx.y
-      const dim3 grid((unsigned)((g.fdim[d][0] * g.fdim[d][1] + 31) / 32), 1u, (unsigned)g.fdim[d][2]);
-      const dim3 blk(32, Cfg<DIM, EQ, NQ>::NQF);
-      if (d == 0) riemann_kernel<DIM, EQ, 0, NQ, SAME><<<grid, blk, 0, s>>>(F[0], G[0], g, sc);
-      if (d == 1) riemann_kernel<DIM, EQ, 1, NQ, SAME><<<grid, blk, 0, s>>>(F[1], G[1], g, sc);
-      if (DIM == 3 && d == 2)
-        riemann_kernel<DIM, EQ, (DIM == 3 ? 2 : 1), NQ, SAME><<<grid, blk, 0, s>>>(F[2], G[2], g, sc);
-    }
-  }
   static cudaError_t riemann(double *const *F, double *const *G, const Grid &g, DevScalars *sc, bool same,
                              cudaStream_t s) {
-    if (same) riemann_dirs<true>(F, G, g, sc, s);
-    else riemann_dirs<false>(F, G, g, sc, s);
+    using R = RiemannShape<DIM, EQ, NQ>;
+    RiemannArgs a;
+    unsigned bx = 0;
+    for (int d = 0; d < DIM; d++) {
+      // consecutive faces of an (x, y) face plane per block (rows of the x faces hold
+      // nx + 1 faces, which would leave a nearly empty block per row)
+      a.F[d] = F[d];
+      a.G[d] = G[d];
+      a.fdiv[d] = ~(uint64_t)0 / (uint64_t)g.fdim[d][0] + 1;
+      a.blocks[d] = (unsigned)((g.fdim[d][0] * g.fdim[d][1] + 32 * R::ROWS - 1) / (32 * R::ROWS));
+      bx = std::max(bx, a.blocks[d]);
+    }
+    const dim3 grid(bx, (unsigned)(g.nz + (DIM == 3 ? 1 : 0)), DIM), blk(32, R::NQF * R::ROWS);
+    if (same) riemann_kernel<DIM, EQ, NQ, true><<<grid, blk, 0, s>>>(a, g, sc);
+    else riemann_kernel<DIM, EQ, NQ, false><<<grid, blk, 0, s>>>(a, g, sc);
     return cudaGetLastError();
   }
   static cudaError_t stage(const StageArgs &a, const Grid &g, cudaStream_t s) {

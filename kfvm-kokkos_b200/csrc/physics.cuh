@@ -58,6 +58,49 @@ __device__ __forceinline__ double rcp_nr(double y) {
   return fma(r, e, r);
 }
 
+// Square root by the coupled Newton iteration for sqrt(x) and 1 / (2 sqrt(x))
+// (Goldschmidt; Markstein 1990) from the hardware's approximate FP64 reciprocal square
+// root: one step, then one correction by the residual x - g^2, within about one ulp.
+// No special-case branches: a negative x gives NaN, values below 1e-290 count as 0.
+__device__ __forceinline__ double sqrt_nr(double x) {
+  double r;
+  asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(x));
+  double g = x * r, h = 0.5 * r;
+  double e = fma(-g, h, 0.5);
+  g = fma(g, e, g);
+  h = fma(h, e, h);
+  e = fma(-g, g, x);
+  g = fma(e, h, g);
+  return fabs(x) < 1e-290 ? 0.0 : g;
+}
+
+// 1 - r^M for r = pMin / pMax in (0, 1]: -expm1(M log r), with log r = 2 atanh(z) and
+// z = (pMin - pMax) / (pMin + pMax).  Where the flow is smooth both series are short
+// (|z| < 0.04: the terms from z^13 on are below 2^-56 of log r; |t| < 1 / 16: those
+// from t^10 on below 2^-58 of t), free of the cancellation in 1 - exp(t), and 15
+// operations instead of a logarithm and an exponential.
+__device__ __forceinline__ double one_minus_pow(double pMin, double pMax, double M) {
+  const double z = (pMin - pMax) * rcp_nr(pMin + pMax), z2 = z * z;
+  double l = fma(z2, 2.0 / 11.0, 2.0 / 9.0);
+  l = fma(z2, l, 2.0 / 7.0);
+  l = fma(z2, l, 2.0 / 5.0);
+  l = fma(z2, l, 2.0 / 3.0);
+  l = fma(z2, l, 2.0);
+  const double t = M * (z * l);
+  if (fabs(z) < 0.04 && fabs(t) < 0.0625 && pMin > 0.0) {
+    double r = fma(t, 1.0 / 362880.0, 1.0 / 40320.0);
+    r = fma(t, r, 1.0 / 5040.0);
+    r = fma(t, r, 1.0 / 720.0);
+    r = fma(t, r, 1.0 / 120.0);
+    r = fma(t, r, 1.0 / 24.0);
+    r = fma(t, r, 1.0 / 6.0);
+    r = fma(t, r, 0.5);
+    r = fma(t, r, 1.0);
+    return -(t * r);
+  }
+  return 1.0 - exp(M * log(fmin(1.0, pMin * rcp_nr(pMax))));
+}
+
 template <int EQ>
 struct Eos {
   static constexpr int NV = EQ == EQ_GLM ? 9 : 5;
@@ -261,21 +304,35 @@ struct Eos {
     return (qL * sqrt(rL) + qR * sqrt(rR)) / (sqrt(rL) + sqrt(rR));
   }
 
+  // GLM-MHD primitives and fast speed with the density reciprocal ir taken once
+  // (fastMagSonic's algebra; pg the pressure)
+  __device__ __forceinline__ static void cons2prim_glm(double g, const double *U, double ir, double *V) {
+    V[0] = U[DENS];
+    V[1] = U[MOMX] * ir;
+    V[2] = U[MOMY] * ir;
+    V[3] = U[MOMZ] * ir;
+    V[4] = (g - 1.0) * eint_r(U, ir);
+  }
+  __device__ __forceinline__ static double fast_r(double g, const double *U, double pg, double ir, double bl) {
+    const double asq = g * pg * ir, absq = asq + 2.0 * prsb(U) * ir, blsq = bl * bl * ir;
+    return sqrt_nr(0.5 * (absq + sqrt_nr(absq * absq - 4.0 * asq * blsq)));
+  }
+
   // GLM-MHD wave-speed estimates (Davis with the cleaning speed, and the Wu-Shu
-  // bound; MHD_GLM_Riemann.H:25-99)
+  // bound; MHD_GLM_Riemann.H:25-99); iL, iR the reciprocal densities
   __device__ __forceinline__ static double speeds(double g, double ch, const int *vo,
                                                   const int *bo, const double *uL,
                                                   const double *uR, const double *vL,
-                                                  const double *vR, double &sL, double &sR) {
-    const double cfL = fastMagSonic(g, uL, uL[bo[0]]);
-    const double cfR = fastMagSonic(g, uR, uR[bo[0]]);
+                                                  const double *vR, double iL, double iR, double &sL, double &sR) {
+    const double cfL = fast_r(g, uL, vL[4], iL, uL[bo[0]]);
+    const double cfR = fast_r(g, uR, vR[4], iR, uR[bo[0]]);
     const double sdL = fmin(vL[vo[0]] - fmax(ch, cfL), vR[vo[0]] - fmax(ch, cfR));
     const double sdR = fmax(vL[vo[0]] + fmax(ch, cfL), vR[vo[0]] + fmax(ch, cfR));
-    const double rtL = sqrt(uL[DENS]), rtR = sqrt(uR[DENS]);
-    const double rtSum = rtL + rtR, vSum = (rtL * vL[vo[0]] + rtR * vR[vo[0]]) / rtSum;
+    const double rtL = sqrt_nr(uL[DENS]), rtR = sqrt_nr(uR[DENS]);
+    const double iSum = rcp_nr(rtL + rtR), vSum = (rtL * vL[vo[0]] + rtR * vR[vo[0]]) * iSum;
     const double b0 = uL[bo[0]] - uR[bo[0]], b1 = uL[bo[1]] - uR[bo[1]],
                  b2 = uL[bo[2]] - uR[bo[2]];
-    const double bnDiff = sqrt(b0 * b0 + b1 * b1 + b2 * b2) / rtSum;
+    const double bnDiff = sqrt_nr(b0 * b0 + b1 * b1 + b2 * b2) * iSum;
     const double aL = fmin(vL[vo[0]], vSum) - cfL - bnDiff;
     const double aR = fmin(vR[vo[0]], vSum) + cfR + bnDiff;
     sL = fmin(sdL, aL);
@@ -293,8 +350,16 @@ struct Eos {
     V[4] = (g - 1.0) * (U[ETOT] - 0.5 * (U[MOMX] * U[MOMX] + U[MOMY] * U[MOMY] + U[MOMZ] * U[MOMZ]) * ir);
   }
 
-  // uL, uR equal to kSameTol (false when either holds a NaN)
+  // uL, uR equal to kSameTol (false when either holds a NaN).  EXACT: equal, which is
+  // what the parity reconstruction gives the two sides of a face in uniform gas.
+  template <bool EXACT>
   __device__ __forceinline__ static bool same_state(const double *uL, const double *uR) {
+    if constexpr (EXACT) {
+      bool eq = true;
+#pragma unroll
+      for (int v = 0; v < NV; v++) eq = eq && uL[v] == uR[v];
+      return eq;
+    }
     double s = 0.0;
 #pragma unroll
     for (int v = 0; v < NV; v++) s = fmax(s, fabs(uL[v]));
@@ -316,9 +381,10 @@ struct Eos {
     const int bo[3] = {MAGX + ord[0], MAGX + ord[1], MAGX + ord[2]};
     if constexpr (EQ == EQ_GLM) {
       double V[NV];
-      cons2prim(g, u, V);
+      const double ir = rcp_nr(u[DENS]);
+      cons2prim_glm(g, u, ir, V);
       flux(ch, vo, bo, u, V, F);
-      return fabs(V[vo[0]]) + fmax(ch, fastMagSonic(g, u, u[bo[0]]));
+      return fabs(V[vo[0]]) + fmax(ch, fast_r(g, u, V[4], ir, u[bo[0]]));
     }
     if constexpr (EQ == EQ_SR) {
       double V[NVP];
@@ -330,20 +396,22 @@ struct Eos {
       const double sm = (V[vo[0]] - rt) / (1.0 + sig), sp = (V[vo[0]] + rt) / (1.0 + sig);
       return fmax(fabs(sm), fabs(sp));
     }
-    const double ir = 1.0 / u[DENS];
+    const double ir = rcp_nr(u[DENS]);
     double V[NV];
     cons2prim_r(g, u, ir, V);
     flux(0.0, vo, bo, u, V, F);
-    return fabs(V[vo[0]]) + sqrt(g * V[4] * ir);
+    return fabs(V[vo[0]]) + sqrt_nr(g * V[4] * ir);
   }
 
   // Riemann solve at one face point in direction dir; returns max(|sL|,|sR|).
   // Euler / Navier-Stokes: Batten/Roe speed estimates (Hydro_Riemann.H:26-80) and,
   // for HLLC, the low-Mach / shear-corrected star fluxes (Hydro_Riemann.H:82-187),
-  // with each repeated divisor (rho, the Roe weight sum, sL - sS, sR - sS, psL - psR)
-  // inverted once by rcp_nr, the Roe weights from one root of rR / rL and the Mach
-  // estimate from one root: 7 reciprocals and 6 roots where the literal form
-  // divides about 30 times.
+  // with each repeated divisor (rho, the Roe weight sum, psL - psR, the star region's
+  // sL - sS or sR - sS) inverted once by rcp_nr, the roots by sqrt_nr, the Roe weights
+  // from one root of rR / rL and the Mach estimate from one root: 7 reciprocals and 6
+  // roots where the literal form divides about 30 times.  The kernel is bound by the
+  // issue rate: the library's square root, logarithm and exponential spent as many
+  // integer and branch instructions on special cases as the FP64 operations proper.
   __device__ __forceinline__ static double solve(int rs, double g, double ch, int dir,
                                                  const double *uL, const double *uR,
                                                  double *F) {
@@ -374,69 +442,63 @@ struct Eos {
       cons2prim_r(g, uR, iR, vR);
       const double pL = vL[4], pR = vR[4];
       const double a2L = g * pL * iL, a2R = g * pR * iR;
-      const double aL = sqrt(a2L), aR = sqrt(a2R);
+      const double aL = sqrt_nr(a2L), aR = sqrt_nr(a2R);
 
       const double hL = (uL[ETOT] + pL) * iL, hR = (uR[ETOT] + pR) * iR;
       // Roe weights sqrt(rL) / (sqrt(rL) + sqrt(rR)) = 1 / (1 + sqrt(rR / rL)) and
       // sqrt(rR) / (...) = sqrt(rR / rL) / (1 + sqrt(rR / rL)): one root, one reciprocal
-      const double tq = sqrt(rR * iL), wL = rcp_nr(1.0 + tq), wR = tq * wL;
+      const double tq = sqrt_nr(rR * iL), wL = rcp_nr(1.0 + tq), wR = tq * wL;
       const double uTil = vL[vo[0]] * wL + vR[vo[0]] * wR, vTil = vL[vo[1]] * wL + vR[vo[1]] * wR,
                    wTil = vL[vo[2]] * wL + vR[vo[2]] * wR, hTil = hL * wL + hR * wR;
       const double vsqTil = uTil * uTil + vTil * vTil + wTil * wTil;
-      const double aTil = sqrt((g - 1.0) * (hTil - 0.5 * vsqTil));
+      const double aTil = sqrt_nr((g - 1.0) * (hTil - 0.5 * vsqTil));
       sL = fmin(vL[vo[0]] - aL, uTil - aTil);
       sR = fmax(vR[vo[0]] + aR, uTil + aTil);
       sMax = fmax(fabs(sL), fabs(sR));
       if (rs == RS_HLLC) {
-        const double vsqL = vL[1] * vL[1] + vL[2] * vL[2] + vL[3] * vL[3];
-        const double vsqR = vR[1] * vR[1] + vR[2] * vR[2] + vR[3] * vR[3];
-        // max of the two Mach numbers max(|v|^2 / a^2) = max(vsqL a2R, vsqR a2L) / (a2L a2R):
-        // one root and one reciprocal of aL aR
-        double M = sqrt(fmax(vsqL * a2R, vsqR * a2L)) * rcp_nr(aL * aR);
         const double uLn = vL[vo[0]], uRn = vR[vo[0]];
         const double psL = rL * (sL - uLn), psR = rR * (sR - uRn);
         // sS and psR psL / (psR - psL) share the reciprocal of psL - psR
         const double iD = rcp_nr(psL - psR);
         const double sS = ((pR - pL) + (psL * uLn - psR * uRn)) * iD;
-        const double pS = 0.5 * ((pL + pR) + psL * (sS - uLn) + psR * (sS - uRn));
-        const double dLR = rcp_nr((sL - sS) * (sR - sS)), dL = (sR - sS) * dLR, dR = (sL - sS) * dLR;
-        const double sFacL = sS * dL, sFacR = sS * dR;
-        const double uJump = uRn - uLn, vJump = vR[vo[1]] - vL[vo[1]], wJump = vR[vo[2]] - vL[vo[2]];
-        const double psiFac = -(psR * psL) * iD;
-        const double presRat = fmin(1.0, fmin(pL, pR) * rcp_nr(fmax(pL, pR)));
-        // presRat^M (pressure ratio in (0, 1]) as exp(M log presRat); exactly 0 for equal pressures
-        const double gFac = pL == pR ? 0.0 : 1.0 - exp(M * log(presRat));
-        const double shFacL = psiFac * gFac * sL * dL, shFacR = psiFac * gFac * sR * dR;
-        M = fmin(M, 1.0);
-        const double omm = 1.0 - M * M;
-        const double fM = M * sqrt(4.0 + omm * omm) * rcp_nr(1.0 + M * M);
-        const double pFacL = psiFac * (fM - 1.0) * uJump + sL * pS * dL;
-        const double pFacR = psiFac * (fM - 1.0) * uJump + sR * pS * dR;
-        if (0 <= sL) {
-          flux(ch, vo, bo, uL, vL, F);
-        } else if (0 <= sS) {
-          flux(ch, vo, bo, uL, vL, F);
-          F[DENS] = sFacL * (sL * uL[DENS] - F[DENS]);
-          F[vo[0]] = sFacL * (sL * uL[vo[0]] - F[vo[0]]) + pFacL;
-          F[vo[1]] = sFacL * (sL * uL[vo[1]] - F[vo[1]]) + shFacL * vJump;
-          F[vo[2]] = sFacL * (sL * uL[vo[2]] - F[vo[2]]) + shFacL * wJump;
-          F[ETOT] = sFacL * (sL * uL[ETOT] - F[ETOT]) + sS * pFacL;
-        } else if (0 < sR) {
-          flux(ch, vo, bo, uR, vR, F);
-          F[DENS] = sFacR * (sR * uR[DENS] - F[DENS]);
-          F[vo[0]] = sFacR * (sR * uR[vo[0]] - F[vo[0]]) + pFacR;
-          F[vo[1]] = sFacR * (sR * uR[vo[1]] - F[vo[1]]) + shFacR * vJump;
-          F[vo[2]] = sFacR * (sR * uR[vo[2]] - F[vo[2]]) + shFacR * wJump;
-          F[ETOT] = sFacR * (sR * uR[ETOT] - F[ETOT]) + sS * pFacR;
-        } else {
-          flux(ch, vo, bo, uR, vR, F);
+        // the side that the face lies on, and whether between its wave and the contact:
+        // one flux for whichever it is, so that the four cases do not split a warp
+        const bool left = 0 <= sL || 0 <= sS, star = left ? !(0 <= sL) : 0 < sR;
+        double u[5], V[5];
+#pragma unroll
+        for (int v = 0; v < 5; v++) {
+          u[v] = left ? uL[v] : uR[v];
+          V[v] = left ? vL[v] : vR[v];
+        }
+        flux(ch, vo, bo, u, V, F);
+        if (star) {
+          const double s = left ? sL : sR;
+          const double vsqL = vL[1] * vL[1] + vL[2] * vL[2] + vL[3] * vL[3];
+          const double vsqR = vR[1] * vR[1] + vR[2] * vR[2] + vR[3] * vR[3];
+          // max of the two Mach numbers max(|v|^2 / a^2) = max(vsqL a2R, vsqR a2L) / (a2L a2R):
+          // one root and one reciprocal of aL aR
+          double M = sqrt_nr(fmax(vsqL * a2R, vsqR * a2L)) * rcp_nr(aL * aR);
+          const double pS = 0.5 * ((pL + pR) + psL * (sS - uLn) + psR * (sS - uRn));
+          const double d = rcp_nr(s - sS), sFac = sS * d;
+          const double psiFac = -(psR * psL) * iD;
+          const double shFac = psiFac * one_minus_pow(fmin(pL, pR), fmax(pL, pR), M) * s * d;
+          M = fmin(M, 1.0);
+          const double omm = 1.0 - M * M;
+          const double fM = M * sqrt_nr(4.0 + omm * omm) * rcp_nr(1.0 + M * M);
+          const double pFac = psiFac * (fM - 1.0) * (uRn - uLn) + s * pS * d;
+          F[DENS] = sFac * (s * u[DENS] - F[DENS]);
+          F[vo[0]] = sFac * (s * u[vo[0]] - F[vo[0]]) + pFac;
+          F[vo[1]] = sFac * (s * u[vo[1]] - F[vo[1]]) + shFac * (vR[vo[1]] - vL[vo[1]]);
+          F[vo[2]] = sFac * (s * u[vo[2]] - F[vo[2]]) + shFac * (vR[vo[2]] - vL[vo[2]]);
+          F[ETOT] = sFac * (s * u[ETOT] - F[ETOT]) + sS * pFac;
         }
         return sMax;
       }
     } else {
-      cons2prim(g, uL, vL);
-      cons2prim(g, uR, vR);
-      sMax = speeds(g, ch, vo, bo, uL, uR, vL, vR, sL, sR);
+      const double iL = rcp_nr(uL[DENS]), iR = rcp_nr(uR[DENS]);
+      cons2prim_glm(g, uL, iL, vL);
+      cons2prim_glm(g, uR, iR, vR);
+      sMax = speeds(g, ch, vo, bo, uL, uR, vL, vR, iL, iR, sL, sR);
     }
     if (rs == RS_LLF) {
       sL = -sMax;
