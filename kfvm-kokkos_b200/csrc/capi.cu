@@ -571,6 +571,12 @@ int eval_front(kfvm_solver *s, int b) {
                                s->W, s->src, s->status, s->lamvel, s->bnd, s->sc, st);
          })) != cudaSuccess)
       return set_err_cuda(e, "recon");
+  } else if ((e = run(s, KFVM_KCLASS_RECON, 1, [&] { return launch_bounds(dim, eq, s->Ub[b], s->g, s->bnd, st); })) !=
+             cudaSuccess) {
+    // WENO everywhere: no reconstruction pass, which would have computed the limiter
+    // bounds (the heavy pass did it per thread: 27 cells' divisions and roots, five times
+    // a cell: 4.2 -> 3.2 ms per evaluation of stirred turbulence 96^3)
+    return set_err_cuda(e, "bounds");
   }
   // the first setFaceBCs of evalRHS: the selector reads the neighbours' states
   if (mode == RECON_SPARSE && !mlpOn)
@@ -597,7 +603,7 @@ int eval_front(kfvm_solver *s, int b) {
     return set_err_cuda(e, "compact");
   if ((e = run(s, KFVM_KCLASS_HEAVY, 1, [&] {
          return launch_heavy(dim, eq, s->Ub[b], s->g, s->dS, s->theta, s->F, s->src, s->heavy,
-                             mode == RECON_FULL ? nullptr : s->bnd, s->sc, jd, s->heavyBlocks, st);
+                             s->bnd, s->sc, jd, s->heavyBlocks, st);
        })) != cudaSuccess)
     return set_err_cuda(e, "heavy");
   if (s->decomposed || s->hasUser) {

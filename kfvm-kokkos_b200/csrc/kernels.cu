@@ -969,9 +969,7 @@ struct HeavyShape {
   static constexpr int NR = LinRows<DIM, EQ, NQ>::NROWS;      // face points, then interior points
   static constexpr int NSUM = T::C + T::CC + T::NB * T::CB;   // stencil cells over all substencils
   static constexpr int NIP = (T::NI + 1) & ~1;                // derivative rows padded to pairs
-  static constexpr int DER = NIP * NSUM;                      // derivative weights [s][p][i]
   static constexpr int NRP = (NR + 1) & ~1;                  // rows padded to pairs
-  static constexpr int FW = NRP * NSUM;                       // reconstruction weights [s][p][row]
   // cells per block (one thread per cell and variable); 16 where 32 cells' rows
   // would not fit in shared memory (3D GLM-MHD with three points: 81 rows x 9)
   static constexpr int CELLS = NR * T::NV > 400 ? 16 : 32;
@@ -983,6 +981,21 @@ struct HeavyShape {
   static constexpr bool MMA = DIM == 3 && (EQ == EQ_HYDRO || EQ == EQ_NS) && NR <= 24 && CELLS == 32;
   static constexpr int MI = (T::NI + 7) / 8;                 // m-tiles of derivative rows
   static constexpr int MR = (NR + 7) / 8;                    // m-tiles of reconstruction rows
+  // the MMA form's K steps of four stencil entries per substencil; its weights are A
+  // fragments [step][m-tile][lane], zero beyond the entries and the rows, so that the
+  // unrolled steps need no bounds and their loads run ahead of the MMAs (with rolled,
+  // guarded steps: 5100 instead of 3600 instructions a warp, 3.2 -> 3.05 ms per evaluation
+  // of stirred turbulence 96^3; bound by the FP64 pipe, 46 % busy, at ten warps per SM)
+  __host__ __device__ static constexpr int ks(int s) { return ((s == 0 ? T::C : (s == 1 ? T::CC : T::CB)) + 3) / 4; }
+  __host__ __device__ static constexpr int ksOff(int s) {
+    return s == 0 ? 0 : (s == 1 ? ks(0) : ks(0) + ks(1) + (s - 2) * ks(2));
+  }
+  static constexpr int KS = ks(0) + ks(1) + T::NB * ks(2);
+  // derivative weights, reconstruction weights: fragments, or [s][p][row] with padded rows
+  static constexpr int DER = MMA ? KS * MI * 32 : NIP * NSUM;
+  static constexpr int FW = MMA ? KS * MR * 32 : NRP * NSUM;
+  // stencil cells of the biased substencils, in the MMA form padded by repeating the first
+  static constexpr int SUB = MMA ? 4 * ks(2) : T::CB;
   static constexpr int VS = 36;                              // row stride of the stencil values [q][cell]
   // cell stride of the row results [cell][row][v], made odd so that the lanes of a
   // warp (its cells) fall on different banks (an even stride of 120 doubles put
@@ -992,7 +1005,7 @@ struct HeavyShape {
   static constexpr int UNION = MMA && T::NV * T::C * VS > CELLS * CS ? T::NV * T::C * VS : CELLS * CS;
   static constexpr int COEF = MMA ? T::NV * T::NSUB * 32 : 0; // [v][s][cell]
   static constexpr size_t BYTES = (size_t)(DER + FW + UNION + CELLS * 2 + CELLS * T::NV + COEF) * sizeof(double) +
-                                  (size_t)T::NB * T::CB * sizeof(int);
+                                  (size_t)T::NB * SUB * sizeof(int);
   __host__ __device__ static constexpr int n(int s) { return s == 0 ? T::C : (s == 1 ? T::CC : T::CB); }
   __host__ __device__ static constexpr int off(int s) {
     return s == 0 ? 0 : (s == 1 ? T::C : T::C + T::CC + (s - 2) * T::CB);
@@ -1020,35 +1033,69 @@ __global__ void __launch_bounds__(HeavyShape<DIM, EQ, NQ>::CELLS * Eos<EQ>::NV, 
   int *sSub = reinterpret_cast<int *>(sCo + H::COEF);
   const kfvm_stencil &st = S->w;
   const int tid = threadIdx.y * H::CELLS + threadIdx.x, nt = H::CELLS * NV;
-  // weights transposed so that the rows of one stencil value are adjacent and
-  // load as 16-byte pairs
-  for (int t = tid; t < H::DER; t += nt) {
-    int s = 0;
-    while (s + 1 < T::NSUB && t >= H::NIP * H::off(s + 1)) s++;
-    const int r = t - H::NIP * H::off(s), p = r / H::NIP, i = r % H::NIP;
-    sDer[t] = i < T::NI ? st.deriv_w[s][i][p] : 0.0;
+  const unsigned count = sc->nheavy;
+  if (blockIdx.x * H::CELLS >= count) return;  // nothing listed for this block: no weights to stage
+  if constexpr (H::MMA) {
+    for (int t = tid; t < (H::MI + H::MR) * H::KS * 32; t += nt) {
+      const bool der = t < H::DER;
+      const int u = der ? t : t - H::DER, m = der ? H::MI : H::MR, l = u % 32, mm = u / 32 % m, kst = u / (32 * m);
+      int s = 0;
+      while (s + 1 < T::NSUB && kst >= H::ksOff(s + 1)) s++;
+      const int p = (kst - H::ksOff(s)) * 4 + (l & 3), row = mm * 8 + (l >> 2);
+      double val = 0.0;
+      if (p < H::n(s)) {
+        if (der) val = row < T::NI ? st.deriv_w[s][row][p] : 0.0;
+        else val = row < NR ? st.face_w[s][row / T::NQF][row % T::NQF][p] : 0.0;  // (no interior points)
+      }
+      sDer[t] = val;
+    }
+  } else {
+    // transposed so that the rows of one stencil value are adjacent and load as
+    // 16-byte pairs
+    for (int t = tid; t < H::DER; t += nt) {
+      int s = 0;
+      while (s + 1 < T::NSUB && t >= H::NIP * H::off(s + 1)) s++;
+      const int r = t - H::NIP * H::off(s), p = r / H::NIP, i = r % H::NIP;
+      sDer[t] = i < T::NI ? st.deriv_w[s][i][p] : 0.0;
+    }
+    for (int t = tid; t < H::FW; t += nt) {
+      int s = 0;
+      while (s + 1 < T::NSUB && t >= H::NRP * H::off(s + 1)) s++;
+      const int r = t - H::NRP * H::off(s), p = r / H::NRP, row = r % H::NRP;
+      const int nfq = T::NF * T::NQF;
+      sFw[t] = row >= NR ? 0.0 : (row < nfq ? st.face_w[s][row / T::NQF][row % T::NQF][p] : st.cell_w[s][row - nfq][p]);
+    }
   }
-  for (int t = tid; t < H::FW; t += nt) {
-    int s = 0;
-    while (s + 1 < T::NSUB && t >= H::NRP * H::off(s + 1)) s++;
-    const int r = t - H::NRP * H::off(s), p = r / H::NRP, row = r % H::NRP;
-    const int nfq = T::NF * T::NQF;
-    sFw[t] = row >= NR ? 0.0 : (row < nfq ? st.face_w[s][row / T::NQF][row % T::NQF][p] : st.cell_w[s][row - nfq][p]);
+  for (int t = tid; t < T::NB * H::SUB; t += nt) {
+    const int q = t % H::SUB;
+    sSub[t] = (int)st.sub_idx[t / H::SUB][q < T::CB ? q : 0];
   }
-  for (int t = tid; t < T::NB * T::CB; t += nt) sSub[t] = (int)st.sub_idx[t / T::CB][t % T::CB];
   __syncthreads();
 
-  const unsigned count = sc->nheavy;
   const int x = threadIdx.x, v = threadIdx.y;
-  double *F[3] = {F0, F1, F2};
   double lam = 0.0, vel = 0.0;
   for (unsigned base = blockIdx.x * H::CELLS; base < count; base += gridDim.x * H::CELLS) {
     const unsigned t = base + x;
     const bool have = t < count;
     const uint32_t e = have ? heavy[t] : 0u;
-    const int64_t c = e & kHeavyCell;
-    const int64_t i = c % g.nx, j = (c / g.nx) % g.ny, k = c / (g.nx * g.ny);
+    // (32-bit divisions: a cell index has 29 bits)
+    const unsigned c = e & kHeavyCell, r1 = c / (unsigned)g.nx, i = c - r1 * (unsigned)g.nx;
+    const unsigned k = r1 / (unsigned)g.ny, j = r1 - k * (unsigned)g.ny;
     const double *Uc = U + pidx(g, i, j, k);
+    // variable v of point 0 of the cell's low face per direction, in the lower slot
+    double *fb[DIM];
+#pragma unroll
+    for (int d = 0; d < DIM; d++)
+      fb[d] = (d == 0 ? F0 : (d == 1 ? F1 : F2)) + v * g.nface[d] + ((k * g.fdim[d][1] + j) * g.fdim[d][0] + i);
+    // row r of the cell where it is stored
+    auto place = [&](int r) {
+      if (r >= T::NF * T::NQF) return src + (((r - T::NF * T::NQF) * NV + v) * g.n + c);
+      const int f = r / T::NQF, q = r % T::NQF, d = f >> 1;
+      const int64_t nf = d == 0 ? g.nface[0] : (d == 1 ? g.nface[1] : g.nface[2]);
+      const int64_t str = d == 0 ? 1 : (d == 1 ? g.fdim[1][0] : g.fdim[2][0] * g.fdim[2][1]);
+      double *b = d == 0 ? fb[0] : (d == 1 ? fb[1] : fb[DIM - 1]);
+      return f & 1 ? b + (q * NV * nf + str) : b + (T::NQF + q) * NV * nf;
+    };
     double *rs = sFs + x * H::CS;
     if constexpr (H::MMA) {
       // ---- WENO-AO with both contractions on the FP64 MMA (mma.sync m8n8k4): warp v
@@ -1093,33 +1140,42 @@ __global__ void __launch_bounds__(HeavyShape<DIM, EQ, NQ>::CELLS * Eos<EQ>::NV, 
           }
         }
         __syncwarp();
-        auto cellOf = [&](int s, int p) { return s < 2 ? p : sSub[(s - 2) * T::CB + p]; };
+        // acc += W_s V_s for the fragments A of substencil s (KST steps, all loads of
+        // the unrolled steps ahead of the MMAs that use them)
+        auto contract = [&](auto kTag, int s, const double *A, double (&acc)[H::MI][4][2]) {
+          constexpr int KST = decltype(kTag)::value;
+          static_assert(H::MI == H::MR, "one accumulator shape");
+#pragma unroll
+          for (int mm = 0; mm < H::MI; mm++)
+#pragma unroll
+            for (int t = 0; t < 4; t++) acc[mm][t][0] = acc[mm][t][1] = 0.0;
+          const double *As = A + H::ksOff(s) * H::MI * 32 + x;
+#pragma unroll
+          for (int ksi = 0; ksi < KST; ksi++) {
+            const int p = 4 * ksi + lq;
+            const int q = s < 2 ? (p < (s == 0 ? T::C : T::CC) ? p : 0) : sSub[(s - 2) * H::SUB + p];
+            double bv[4], av[H::MI];
+#pragma unroll
+            for (int t = 0; t < 4; t++) bv[t] = sVw[q * H::VS + 8 * t + ln];
+#pragma unroll
+            for (int mm = 0; mm < H::MI; mm++) av[mm] = As[(ksi * H::MI + mm) * 32];
+#pragma unroll
+            for (int mm = 0; mm < H::MI; mm++)
+#pragma unroll
+              for (int t = 0; t < 4; t++) dmma_884(acc[mm][t], av[mm], bv[t]);
+          }
+        };
+        auto substencil = [&](int s, const double *A, double (&acc)[H::MI][4][2]) {
+          if (s == 0) contract(std::integral_constant<int, H::ks(0)>{}, 0, A, acc);
+          else if (s == 1) contract(std::integral_constant<int, H::ks(1)>{}, 1, A, acc);
+          else contract(std::integral_constant<int, H::ks(2)>{}, s, A, acc);
+        };
         // smoothness indicators: b = D_s V_s per substencil, beta = sum of b^2 over
         // the rows (lane l holds rows 8 m + l / 4 of cells 8 t + 2 (l % 4) + e)
 #pragma unroll 1
         for (int s = 0; s < T::NSUB; s++) {
-          const int n = H::n(s);
-          const double *D = sDer + H::NIP * H::off(s);
           double bd[H::MI][4][2];
-#pragma unroll
-          for (int mm = 0; mm < H::MI; mm++)
-#pragma unroll
-            for (int t = 0; t < 4; t++) bd[mm][t][0] = bd[mm][t][1] = 0.0;
-          for (int p0 = 0; p0 < n; p0 += 4) {
-            const int p = p0 + lq;
-            const bool pk = p < n;
-            const int q = pk ? cellOf(s, p) : 0;
-            double bv[4];
-#pragma unroll
-            for (int t = 0; t < 4; t++) bv[t] = pk ? sVw[q * H::VS + 8 * t + ln] : 0.0;
-#pragma unroll
-            for (int mm = 0; mm < H::MI; mm++) {
-              const int row = 8 * mm + ln;
-              const double av = pk && row < T::NI ? D[p * H::NIP + row] : 0.0;
-#pragma unroll
-              for (int t = 0; t < 4; t++) dmma_884(bd[mm][t], av, bv[t]);
-            }
-          }
+          substencil(s, sDer, bd);
 #pragma unroll
           for (int t = 0; t < 4; t++)
 #pragma unroll
@@ -1184,28 +1240,8 @@ __global__ void __launch_bounds__(HeavyShape<DIM, EQ, NQ>::CELLS * Eos<EQ>::NV, 
           for (int t = 0; t < 4; t++) acc[mm][t][0] = acc[mm][t][1] = 0.0;
 #pragma unroll 1
         for (int s = 0; s < T::NSUB; s++) {
-          const int n = H::n(s);
-          const double *Wr = sFw + H::NRP * H::off(s);
           double tt[H::MR][4][2];
-#pragma unroll
-          for (int mm = 0; mm < H::MR; mm++)
-#pragma unroll
-            for (int t = 0; t < 4; t++) tt[mm][t][0] = tt[mm][t][1] = 0.0;
-          for (int p0 = 0; p0 < n; p0 += 4) {
-            const int p = p0 + lq;
-            const bool pk = p < n;
-            const int q = pk ? cellOf(s, p) : 0;
-            double bv[4];
-#pragma unroll
-            for (int t = 0; t < 4; t++) bv[t] = pk ? sVw[q * H::VS + 8 * t + ln] : 0.0;
-#pragma unroll
-            for (int mm = 0; mm < H::MR; mm++) {
-              const int row = 8 * mm + ln;
-              const double av = pk && row < NR ? Wr[p * H::NRP + row] : 0.0;
-#pragma unroll
-              for (int t = 0; t < 4; t++) dmma_884(tt[mm][t], av, bv[t]);
-            }
-          }
+          substencil(s, sFw, tt);
 #pragma unroll
           for (int t = 0; t < 4; t++)
 #pragma unroll
@@ -1359,16 +1395,8 @@ __global__ void __launch_bounds__(HeavyShape<DIM, EQ, NQ>::CELLS * Eos<EQ>::NV, 
     }
     auto load_linear = [&]() {
       // the linear states the reconstruction pass wrote
-      for (int r = 0; r < NR; r++) {
-        double val;
-        if (r < T::NF * T::NQF) {
-          const int f = r / T::NQF, q = r % T::NQF;
-          val = F[f >> 1][face_slot_addr(g, f, i, j, k, q, v, T::NQF, NV)];
-        } else {
-          val = src[((r - T::NF * T::NQF) * NV + v) * g.n + c];
-        }
-        rs[r * NV + v] = val;
-      }
+#pragma unroll
+      for (int r = 0; r < NR; r++) rs[r * NV + v] = *place(r);
     };
     if (have && !(e & kHeavyWeno)) load_linear();  // limiter only
     __syncthreads();
@@ -1399,15 +1427,10 @@ __global__ void __launch_bounds__(HeavyShape<DIM, EQ, NQ>::CELLS * Eos<EQ>::NV, 
         if (lab && !p) atomicAdd(&sc->mlp_missed, 1ull);
         if (!lab && p) atomicAdd(&sc->mlp_false, 1ull);
       }
-      if (bnd) {
-        // the reconstruction pass computed them (pos_bounds_tile)
-        bd.rDens = ref[DENS];
-        bd.minDens = bnd[c];
-        bd.maxDens = bnd[g.n + c];
-        bd.minEint = bnd[2 * g.n + c];
-      } else {
-        bd = pos_bounds<DIM, EQ>(Uc, g);
-      }
+      bd.rDens = ref[DENS];
+      bd.minDens = bnd[c];
+      bd.maxDens = bnd[g.n + c];
+      bd.minEint = bnd[2 * g.n + c];
     }
     const double rDens = bd.rDens, minDens = bd.minDens, maxDens = bd.maxDens, minEint = bd.minEint;
     const double rDP = maxDens - rDens, rDM = rDens - minDens;
@@ -1461,7 +1484,7 @@ __global__ void __launch_bounds__(HeavyShape<DIM, EQ, NQ>::CELLS * Eos<EQ>::NV, 
           double st[NV];
 #pragma unroll
           for (int w = 0; w < NV; w++) st[w] = rs[r * NV + w];
-          if (!(E::eint(st) > minEint)) {
+          if (!(E::eint_vs(st, minEint) > minEint)) {
             double a = 0.0, b = 1.0;
             for (int itb = 0; itb < 10; itb++) {
               const double cm = 0.5 * (a + b);
@@ -1498,15 +1521,8 @@ __global__ void __launch_bounds__(HeavyShape<DIM, EQ, NQ>::CELLS * Eos<EQ>::NV, 
     __syncthreads();
     // stores: thread (cell, v) writes variable v of every row
     if (have) {
-      for (int r = 0; r < NR; r++) {
-        const double val = rs[r * NV + v];
-        if (r < T::NF * T::NQF) {
-          const int f = r / T::NQF, q = r % T::NQF;
-          F[f >> 1][face_slot_addr(g, f, i, j, k, q, v, T::NQF, NV)] = val;
-        } else {
-          src[((r - T::NF * T::NQF) * NV + v) * g.n + c] = val;
-        }
-      }
+#pragma unroll
+      for (int r = 0; r < NR; r++) *place(r) = rs[r * NV + v];
     }
     __syncthreads();
   }

@@ -102,8 +102,7 @@ cudaError_t launch_flag(int dim, int eq, const double *U, const Grid &g, float *
 cudaError_t launch_compact(int dim, int eq, const Grid &g, int mode, const uint8_t *flag, uint8_t *wset,
                            const uint8_t *status, uint8_t *applied, double *theta, uint32_t *heavy,
                            const double2 *lamvel, DevScalars *sc, const JudgeArgs &jd, cudaStream_t s);
-// bnd: the reconstruction's limiter bounds, or null (full-WENO evaluations, where
-// no reconstruction pass ran) to compute them from the state
+// bnd: the limiter bounds (the reconstruction's, or launch_bounds' where WENO runs everywhere)
 cudaError_t launch_heavy(int dim, int eq, const double *U, const Grid &g, const DevStencil *S,
                          double *theta, double *const *F, double *src, const uint32_t *heavy,
                          const double *bnd, DevScalars *sc, const JudgeArgs &jd, int heavy_blocks,
