@@ -442,14 +442,15 @@ int reduce_all(kfvm_solver *s, int op, double *vals, int n) {
   return KFVM_OK;
 }
 
-// the halo of buffer b: one launch on one domain; on a decomposed domain axis by
+// the halo of buffer b: one launch on one domain (which also resets the evaluation's
+// counters in `reset`, if given); on a decomposed domain axis by
 // axis, exchange faces from the neighbours, the others from this block
-int fill_halo(kfvm_solver *s, int b) {
+int fill_halo(kfvm_solver *s, int b, kfvm::DevScalars *reset = nullptr) {
   using namespace kfvm;
   cudaStream_t st = s->stream;
   double *U = s->Ub[b];
   if (!s->decomposed && !s->hasUser) {
-    cudaError_t e = run(s, KFVM_KCLASS_BC, 1, [&] { return launch_bc(s->dim, s->eq, U, s->g, st); });
+    cudaError_t e = run(s, KFVM_KCLASS_BC, 1, [&] { return launch_bc(s->dim, s->eq, U, s->g, reset, st); });
     return e == cudaSuccess ? KFVM_OK : set_err_cuda(e, "bc");
   }
   if (s->decomposed && !s->xfn) return fail(KFVM_ERR_STATE, "exchange faces but no transport (kfvm_set_exchange)");
@@ -536,9 +537,11 @@ int eval_front(kfvm_solver *s, int b) {
   cudaStream_t st = s->stream;
   const int dim = s->dim, eq = s->eq;
   cudaError_t e;
-  if (int rc = fill_halo(s, b)) return rc;
+  if (int rc = fill_halo(s, b, s->sc)) return rc;
   // reset the per-evaluation counters (nflag, napplied, nheavy) and the GLM maxima
-  CK(cudaMemsetAsync(&s->sc->glm_lam_bits, 0, 2 * sizeof(unsigned long long) + 3 * sizeof(unsigned), st));
+  // (launch_bc did, where it filled the halo)
+  if (s->decomposed || s->hasUser)
+    CK(cudaMemsetAsync(&s->sc->glm_lam_bits, 0, 2 * sizeof(unsigned long long) + 3 * sizeof(unsigned), st));
   int mode;
   if (s->indicator == KFVM_IND_NONE) {
     mode = RECON_LINEAR;
@@ -971,6 +974,7 @@ int kfvm_create(const kfvm_config *cfg, kfvm_solver **out) {
   g.gamma = cfg->gamma;
   g.rs = cfg->rs;
   g.nq = cfg->nq;
+  g.chain = cfg->dim == 2 || g.n <= (1 << 16);
   s->dmin = cfg->dim == 2 ? std::fmin(g.dx, g.dy) : std::fmin(g.dx, std::fmin(g.dy, g.dz));
 
   DevStencil hS;

@@ -25,49 +25,55 @@ __device__ __forceinline__ int64_t axis_map(int64_t i, int64_t n, int bcLo, int 
   return i;
 }
 
+// The first kernel of an evaluation: it also resets the evaluation's counters and GLM
+// maxima (sc, if given).  32-bit indices: the halo has fewer than 2^32 cells, and the chain of
+// 64-bit divisions took longer than the copies (8 -> 4 us at 32^2).
 template <int DIM, int NV>
-__global__ void __launch_bounds__(256) bc_fill_kernel(double *__restrict__ U, Grid g) {
-  const int64_t r = kRad;
-  const int64_t hx = g.nx + 2 * r, hy = g.ny + 2 * r;
-  const int64_t nxs = 2 * r * g.ny * g.nz;                 // x slabs (interior y,z)
-  const int64_t nys = hx * 2 * r * g.nz;                   // y slabs (all x, interior z)
-  const int64_t nzs = DIM == 3 ? hx * hy * 2 * r : 0;      // z slabs (all x, y)
-  const int64_t total = nxs + nys + nzs;
-  for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < total;
-       t += (int64_t)gridDim.x * blockDim.x) {
-    int64_t i, j, k;
-    if (t < nxs) {
-      const int64_t a = t % (2 * r), b = t / (2 * r);
-      i = a < r ? a - r : g.nx + (a - r);
-      j = b % g.ny;
-      k = b / g.ny;
-    } else if (t < nxs + nys) {
-      const int64_t u = t - nxs, a = u % hx, b = u / hx;
-      i = a - r;
-      const int64_t jj = b % (2 * r);
-      j = jj < r ? jj - r : g.ny + (jj - r);
-      k = b / (2 * r);
-    } else {
-      const int64_t u = t - nxs - nys, a = u % hx, b = u / hx;
-      i = a - r;
-      j = b % hy - r;
-      const int64_t kk = b / hy;
-      k = kk < r ? kk - r : g.nz + (kk - r);
-    }
-    const int64_t si = axis_map(i, g.nx, g.bc[0], g.bc[1]);
-    const int64_t sj = axis_map(j, g.ny, g.bc[2], g.bc[3]);
-    const int64_t sk = DIM == 3 ? axis_map(k, g.nz, g.bc[4], g.bc[5]) : k;
-    const int64_t dst = pidx(g, i, j, k), src = pidx(g, si, sj, sk);
-    // wall mirrors flip signs; the sequential x, y, z fills of the reference
-    // multiply a corner by the coefficients of every wall it lies beyond
-    unsigned flip = (i < 0 ? g.bflip[0] : (i >= g.nx ? g.bflip[1] : 0u)) ^
-                    (j < 0 ? g.bflip[2] : (j >= g.ny ? g.bflip[3] : 0u));
-    if (DIM == 3) flip ^= k < 0 ? g.bflip[4] : (k >= g.nz ? g.bflip[5] : 0u);
+__global__ void __launch_bounds__(256)
+    bc_fill_kernel(double *__restrict__ U, const __grid_constant__ Grid g, DevScalars *__restrict__ sc) {
+  pdl_begin();
+  if (sc && blockIdx.x == 0 && threadIdx.x == 0) {
+    sc->glm_lam_bits = sc->glm_vel_bits = 0ull;
+    sc->nflag = sc->napplied = sc->nheavy = 0u;
+  }
+  constexpr unsigned r = kRad;
+  const unsigned nx = (unsigned)g.nx, ny = (unsigned)g.ny, nz = (unsigned)g.nz;
+  const unsigned hx = nx + 2 * r, hy = ny + 2 * r;
+  const unsigned nxs = 2 * r * ny * nz;              // x slabs (interior y,z)
+  const unsigned nys = hx * 2 * r * nz;              // y slabs (all x, interior z)
+  const unsigned nzs = DIM == 3 ? hx * hy * 2 * r : 0;  // z slabs (all x, y)
+  const unsigned t = blockIdx.x * 256u + threadIdx.x;
+  if (t >= nxs + nys + nzs) return;
+  int i, j, k;
+  if (t < nxs) {
+    const unsigned a = t % (2 * r), b = t / (2 * r);
+    k = (int)(b / ny);
+    j = (int)(b - (unsigned)k * ny);
+    i = a < r ? (int)a - (int)r : (int)(nx + (a - r));
+  } else if (t < nxs + nys) {
+    const unsigned u = t - nxs, b = u / hx, jj = b % (2 * r);
+    i = (int)(u - b * hx) - (int)r;
+    j = jj < r ? (int)jj - (int)r : (int)(ny + (jj - r));
+    k = (int)(b / (2 * r));
+  } else {
+    const unsigned u = t - nxs - nys, b = u / hx, kk = b / hy;
+    i = (int)(u - b * hx) - (int)r;
+    j = (int)(b - kk * hy) - (int)r;
+    k = kk < r ? (int)kk - (int)r : (int)(nz + (kk - r));
+  }
+  const int64_t si = axis_map(i, g.nx, g.bc[0], g.bc[1]);
+  const int64_t sj = axis_map(j, g.ny, g.bc[2], g.bc[3]);
+  const int64_t sk = DIM == 3 ? axis_map(k, g.nz, g.bc[4], g.bc[5]) : k;
+  const int64_t dst = pidx(g, i, j, k), src = pidx(g, si, sj, sk);
+  // wall mirrors flip signs; the sequential x, y, z fills of the reference
+  // multiply a corner by the coefficients of every wall it lies beyond
+  unsigned flip = (i < 0 ? g.bflip[0] : (i >= g.nx ? g.bflip[1] : 0u)) ^
+                  (j < 0 ? g.bflip[2] : (j >= g.ny ? g.bflip[3] : 0u));
+  if (DIM == 3) flip ^= k < 0 ? g.bflip[4] : (k >= g.nz ? g.bflip[5] : 0u);
 #pragma unroll
-    for (int v = 0; v < NV; v++) {
-      const double x = U[v * g.pvol + src];
-      U[v * g.pvol + dst] = (flip >> v) & 1u ? -x : x;
-    }
+  for (int v = 0; v < NV; v++) {
+    const double x = U[v * g.pvol + src];
+    U[v * g.pvol + dst] = (flip >> v) & 1u ? -x : x;
   }
 }
 
@@ -380,6 +386,7 @@ __global__ void __launch_bounds__(DmmaTile<DIM>::THREADS, (DIM == 2 && NQ == 2 &
   using T = Cfg<DIM, EQ, NQ>;
   using Sh = DmmaShape<DIM, EQ, NQ>;
   using D = DmmaTile<DIM>;
+  pdl_begin();
   using L = DmmaTmaSmem<DIM, EQ, NQ>;
   using E = Eos<EQ>;
   constexpr int NV = T::NV, NT = Sh::NT, NK = Sh::NK;
@@ -813,6 +820,7 @@ __global__ void __launch_bounds__(128, 8)
                 const double *__restrict__ F0, const double *__restrict__ F1,
                 const double *__restrict__ F2, const double *__restrict__ theta,
                 uint8_t *__restrict__ flag, DevScalars *__restrict__ sc, double wThresh) {
+  pdl_begin();
   using T = Cfg<DIM, EQ, NQ>;
   constexpr int NV = T::NV;
   const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
@@ -821,8 +829,9 @@ __global__ void __launch_bounds__(128, 8)
   bool f = false;
   if (i < g.nx && j < g.ny) {
     const int64_t c = (k * g.ny + j) * g.nx + i;
-    f = theta[c] < 1.0;
-    if (!f) {
+    // every load is issued at once, also for the few cells that theta flags already
+    const bool limited = theta[c] < 1.0;
+    {
       double uAv[NV];
       const double *Uc = U + pidx(g, i, j, k);
 #pragma unroll
@@ -880,7 +889,8 @@ __global__ void __launch_bounds__(128, 8)
           certain = true;
         }
       }
-      if (!certain) {
+      f = f || limited;
+      if (!certain && !limited) {
         const double *F[3] = {F0, F1, F2};
         double maxJump = 0.0;
         for (int fc = 0; fc < T::NF; fc++) {
@@ -918,6 +928,7 @@ __global__ void __launch_bounds__(256)
                    const uint8_t *__restrict__ status, uint8_t *__restrict__ applied,
                    double *__restrict__ theta, uint32_t *__restrict__ heavy,
                    const double2 *__restrict__ lamvel, DevScalars *__restrict__ sc, JudgeArgs jd) {
+  pdl_begin();
   const int64_t c = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   bool useWeno = false, push = false, judged = false, judgeOnly = false;
   double lam = 0.0, vel = 0.0;
@@ -1038,6 +1049,7 @@ __global__ void __launch_bounds__(HeavyShape<DIM, EQ, NQ>::CELLS * Eos<EQ>::NV, 
                      double *__restrict__ theta, double *__restrict__ F0, double *__restrict__ F1,
                      double *__restrict__ F2, double *__restrict__ src, const uint32_t *__restrict__ heavy,
                      const double *__restrict__ bnd, DevScalars *__restrict__ sc, JudgeArgs jd) {
+  pdl_begin();
   using T = Cfg<DIM, EQ, NQ>;
   using H = HeavyShape<DIM, EQ, NQ>;
   using E = Eos<EQ>;
@@ -1709,6 +1721,7 @@ struct RiemannArgs {
 template <int DIM, int EQ, int NQ, bool SAME>
 __global__ void __launch_bounds__(RiemannShape<DIM, EQ, NQ>::THREADS, RiemannShape<DIM, EQ, NQ>::RESIDENT)
     riemann_kernel(const __grid_constant__ RiemannArgs a, const __grid_constant__ Grid g, DevScalars *__restrict__ sc) {
+  pdl_begin();
   using R = RiemannShape<DIM, EQ, NQ>;
   __shared__ double part[R::ROWS][R::NQF][Eos<EQ>::NV][32];
   __shared__ unsigned cnt[2];
@@ -2003,6 +2016,7 @@ __global__ void __launch_bounds__(128)
                  const double *__restrict__ src, const double *__restrict__ theta, int mode,
                  StageCoef co, double Re, double Pr, double atol, double rtol,
                  double *__restrict__ part) {
+  pdl_begin();
   using T = Cfg<DIM, EQ, NQ>;
   using E = Eos<EQ>;
   constexpr int NV = T::NV;
@@ -2125,6 +2139,7 @@ __global__ void __launch_bounds__(128)
 // fixed-order sum of the block partials (one block)
 __global__ void __launch_bounds__(1024) finalize_kernel(const double *__restrict__ part,
                                                          int64_t nblk, DevScalars *sc) {
+  pdl_begin();
   __shared__ double se[1024], sp[1024];
   double a = 0.0, b = 1.0;
   for (int64_t t = threadIdx.x; t < nblk; t += blockDim.x) {
@@ -2154,6 +2169,7 @@ __global__ void __launch_bounds__(128)
                      double *__restrict__ Uhat, double *__restrict__ Utmp,
                      const double *__restrict__ K, Grid g, double betaDt, double bhatDt,
                      int use_tmp) {
+  pdl_begin();
   const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   const int64_t j = blockIdx.y * (int64_t)blockDim.y + threadIdx.y;
   const int64_t k = blockIdx.z;
@@ -2191,12 +2207,10 @@ static dim3 cell_grid(const Grid &g) {
 template <int DIM, int EQ, int NQ>
 struct Launch {
   static constexpr int NV = Eos<EQ>::NV;
-  static cudaError_t bc(double *U, const Grid &g, cudaStream_t s) {
+  static cudaError_t bc(double *U, const Grid &g, DevScalars *sc, cudaStream_t s) {
     const int64_t r = kRad, hx = g.nx + 2 * r, hy = g.ny + 2 * r;
     const int64_t total = 2 * r * g.ny * g.nz + hx * 2 * r * g.nz + (DIM == 3 ? hx * hy * 2 * r : 0);
-    const int64_t blocks = (total + 255) / 256;
-    bc_fill_kernel<DIM, NV><<<(unsigned)(blocks < 65535 * 16 ? blocks : 65535 * 16), 256, 0, s>>>(U, g);
-    return cudaGetLastError();
+    return launch_chain(g.chain, bc_fill_kernel<DIM, NV>, dim3((unsigned)((total + 255) / 256)), dim3(256), 0, s, U, g, sc);
   }
   static cudaError_t bounds(const double *U, const Grid &g, double *bnd, cudaStream_t s) {
     if constexpr (DIM == 3) {
@@ -2236,9 +2250,8 @@ struct Launch {
         if (attr != cudaSuccess) return attr;
         const dim3 grid((unsigned)((g.nx + D::BX - 1) / D::BX), (unsigned)((g.ny + D::BY - 1) / D::BY),
                         (unsigned)((g.nz + D::BZ - 1) / D::BZ));
-        recon_tma_kernel<DIM, EQ, NQ><<<grid, D::THREADS, L::BYTES, s>>>(
-            *umap, g, S, wantInd, F[0], F[1], F[2], W[0], W[1], W[2], src, status, lamvel, bnd, sc);
-        return cudaGetLastError();
+        return launch_chain(g.chain, recon_tma_kernel<DIM, EQ, NQ>, grid, dim3(D::THREADS), L::BYTES, s, *umap, g, S, wantInd,
+                            F[0], F[1], F[2], W[0], W[1], W[2], src, status, lamvel, bnd, sc);
       }
     }
     recon_kernel<DIM, EQ, NQ><<<cell_grid(g), dim3(kBlockX, kBlockY), 0, s>>>(
@@ -2248,16 +2261,14 @@ struct Launch {
   }
   static cudaError_t flag(const double *U, const Grid &g, float *const *W, double *const *F,
                           const double *theta, uint8_t *flag, DevScalars *sc, double thr, cudaStream_t s) {
-    flag_kernel<DIM, EQ, NQ><<<cell_grid(g), dim3(kBlockX, kBlockY), 0, s>>>(U, g, W[0], W[1], W[2], F[0], F[1],
-                                                                          F[2], theta, flag, sc, thr);
-    return cudaGetLastError();
+    return launch_chain(g.chain, flag_kernel<DIM, EQ, NQ>, cell_grid(g), dim3(kBlockX, kBlockY), 0, s, U, g, W[0], W[1], W[2],
+                        F[0], F[1], F[2], theta, flag, sc, thr);
   }
   static cudaError_t compact(const Grid &g, int mode, const uint8_t *flag, uint8_t *wset,
                              const uint8_t *status, uint8_t *applied, double *theta, uint32_t *heavy,
                              const double2 *lamvel, DevScalars *sc, const JudgeArgs &jd, cudaStream_t s) {
-    compact_kernel<DIM, EQ><<<(unsigned)((g.n + 255) / 256), 256, 0, s>>>(g, mode, flag, wset, status, applied,
-                                                                           theta, heavy, lamvel, sc, jd);
-    return cudaGetLastError();
+    return launch_chain(g.chain, compact_kernel<DIM, EQ>, dim3((unsigned)((g.n + 255) / 256)), dim3(256), 0, s, g, mode, flag,
+                        wset, status, applied, theta, heavy, lamvel, sc, jd);
   }
   static cudaError_t heavy(const double *U, const Grid &g, const DevStencil *S, double *theta,
                            double *const *F, double *src, const uint32_t *heavy, const double *bnd,
@@ -2267,9 +2278,9 @@ struct Launch {
     static const cudaError_t attr = cudaFuncSetAttribute(
         heavy_var_kernel<DIM, EQ, NQ>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)HeavyShape<DIM, EQ, NQ>::BYTES);
     if (attr != cudaSuccess) return attr;
-    heavy_var_kernel<DIM, EQ, NQ><<<heavy_blocks, dim3(HeavyShape<DIM, EQ, NQ>::CELLS, NV), HeavyShape<DIM, EQ, NQ>::BYTES, s>>>(
-        U, g, S, theta, F[0], F[1], F[2], src, heavy, bnd, sc, jd);
-    return cudaGetLastError();
+    using H = HeavyShape<DIM, EQ, NQ>;
+    return launch_chain(g.chain, heavy_var_kernel<DIM, EQ, NQ>, dim3(heavy_blocks), dim3(H::CELLS, NV), H::BYTES, s, U, g, S,
+                        theta, F[0], F[1], F[2], src, heavy, bnd, sc, jd);
   }
   static cudaError_t riemann(double *const *F, double *const *G, const Grid &g, DevScalars *sc, bool same,
                              cudaStream_t s) {
@@ -2286,27 +2297,22 @@ struct Launch {
       bx = std::max(bx, a.blocks[d]);
     }
     const dim3 grid(bx, (unsigned)(g.nz + (DIM == 3 ? 1 : 0)), DIM), blk(32, R::NQF * R::ROWS);
-    if (same) riemann_kernel<DIM, EQ, NQ, true><<<grid, blk, 0, s>>>(a, g, sc);
-    else riemann_kernel<DIM, EQ, NQ, false><<<grid, blk, 0, s>>>(a, g, sc);
-    return cudaGetLastError();
+    return same ? launch_chain(g.chain, riemann_kernel<DIM, EQ, NQ, true>, grid, blk, 0, s, a, g, sc)
+                : launch_chain(g.chain, riemann_kernel<DIM, EQ, NQ, false>, grid, blk, 0, s, a, g, sc);
   }
   static cudaError_t stage(const StageArgs &a, const Grid &g, cudaStream_t s) {
     const dim3 grid = cell_grid(g);
-    stage_kernel<DIM, EQ, NQ><<<grid, dim3(kBlockX, kBlockY), 0, s>>>(
-        a.U, a.Unext, a.Uprev, a.Uhat, a.Utmp, a.K, g, a.G[0], a.G[1], a.G[2], a.F[0], a.F[1],
-        a.F[2], a.src, a.theta, a.mode, a.co, a.Re, a.Pr, a.atol, a.rtol, a.part);
-    if (a.mode == STAGE_FSAL) {
-      const int64_t nblk = (int64_t)grid.x * grid.y * grid.z;
-      finalize_kernel<<<1, 1024, 0, s>>>(a.part, nblk, a.sc);
-    }
-    return cudaGetLastError();
+    const cudaError_t e = launch_chain(g.chain, stage_kernel<DIM, EQ, NQ>, grid, dim3(kBlockX, kBlockY), 0, s, a.U, a.Unext,
+                                       a.Uprev, a.Uhat, a.Utmp, a.K, g, a.G[0], a.G[1], a.G[2], a.F[0], a.F[1], a.F[2],
+                                       a.src, a.theta, a.mode, a.co, a.Re, a.Pr, a.atol, a.rtol, a.part);
+    if (e != cudaSuccess || a.mode != STAGE_FSAL) return e;
+    return launch_chain(g.chain, finalize_kernel, dim3(1), dim3(1024), 0, s, a.part, (int64_t)grid.x * grid.y * grid.z, a.sc);
   }
   static cudaError_t stage_pre(double *U1, const double *Uprev, double *Uhat, double *Utmp,
                                const double *K, const Grid &g, double betaDt, double bhatDt,
                                int use_tmp, cudaStream_t s) {
-    stage_pre_kernel<NV><<<cell_grid(g), dim3(kBlockX, kBlockY), 0, s>>>(U1, Uprev, Uhat, Utmp, K, g,
-                                                                          betaDt, bhatDt, use_tmp);
-    return cudaGetLastError();
+    return launch_chain(g.chain, stage_pre_kernel<NV>, cell_grid(g), dim3(kBlockX, kBlockY), 0, s, U1, Uprev, Uhat, Utmp, K, g,
+                        betaDt, bhatDt, use_tmp);
   }
   static cudaError_t copy(double *dst, const double *src, const Grid &g, cudaStream_t s) {
     copy_interior_kernel<NV><<<cell_grid(g), dim3(kBlockX, kBlockY), 0, s>>>(dst, src, g);
@@ -2418,8 +2424,8 @@ cudaError_t launch_fill(double *p, int64_t n, double val, cudaStream_t s) {
   return cudaGetLastError();
 }
 
-cudaError_t launch_bc(int dim, int eq, double *U, const Grid &g, cudaStream_t s) {
-  KFVM_DISPATCH(dim, eq, bc(U, g, s));
+cudaError_t launch_bc(int dim, int eq, double *U, const Grid &g, DevScalars *sc, cudaStream_t s) {
+  KFVM_DISPATCH(dim, eq, bc(U, g, sc, s));
 }
 cudaError_t launch_bounds(int dim, int eq, const double *U, const Grid &g, double *bnd, cudaStream_t s) {
   KFVM_DISPATCH(dim, eq, bounds(U, g, bnd, s));

@@ -46,6 +46,7 @@ struct Grid {
   double dx, dy, dz;
   double rdx, rdy, rdz;      // 1 / dx, 1 / dy, 1 / dz
   int nq;                    // Gauss points per direction
+  bool chain;                // kernels of an evaluation start early (launch_chain)
   int bc[6];
   // variables whose sign the wall mirror flips, bit v per face (reflecting and
   // no-slip coefficient tables of <Eq>_BCCoeffs.H; 0 for periodic / outflow)
@@ -130,6 +131,13 @@ struct StageCoef {
   double delta, g1, g2, g3, betaDt, bhatDt;
   int use_tmp; // delta or g2 nonzero somewhere in the scheme
 };
+
+// The start of a kernel launched by launch_chain: lets the next one of the chain be
+// launched, and waits until the previous one has completed and its writes are visible.
+__device__ __forceinline__ void pdl_begin() {
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+}
 
 __device__ __forceinline__ int64_t pidx(const Grid &g, int64_t i, int64_t j, int64_t k) {
   return ((k + g.rz) * g.py + (j + kRad)) * g.px + (i + kRad);

@@ -427,6 +427,7 @@ __global__ void __launch_bounds__(Sym3<EQ>::THREADS, Sym3<EQ>::RESIDENT)
                       float *__restrict__ W0, float *__restrict__ W1, float *__restrict__ W2,
                       double *__restrict__ src, uint8_t *__restrict__ status, double2 *__restrict__ lamvel,
                       double *__restrict__ bnd, DevScalars *__restrict__ sc) {
+  pdl_begin();
   using L = Sym3<EQ>;
   using E = Eos<EQ>;
   constexpr int NV = L::NV, TX = L::TX, TN = L::TN, PX = L::PX, PN = L::PN, NQF = 4;
@@ -715,6 +716,7 @@ __global__ void __launch_bounds__(Sym2<EQ>::THREADS, Sym2<EQ>::RESIDENT)
                       float *__restrict__ W0, float *__restrict__ W1, double *__restrict__ src,
                       uint8_t *__restrict__ status, double2 *__restrict__ lamvel, double *__restrict__ bnd,
                       DevScalars *__restrict__ sc) {
+  pdl_begin();
   using L = Sym2<EQ>;
   constexpr int NV = L::NV, TX = L::TX, TN = L::TN, PX = L::PX, PN = L::PN;
   __shared__ __align__(128) double tile[NV * TN];
@@ -873,19 +875,16 @@ static cudaError_t sym3(const ReconSymArgs &a, const CUtensorMap &umap, const Gr
       off.w[d][o] = q * g.nface[d] + str;
     }
   const dim3 grid((unsigned)bx, (unsigned)by, (unsigned)((g.nz + zc - 1) / zc));
-  recon_sym3_kernel<EQ><<<grid, L::THREADS, L::BYTES, s>>>(umap, g, w, off, (int)zc, a.wantInd, a.F[0], a.F[1], a.F[2],
-                                                         a.W[0], a.W[1], a.W[2], a.src, a.status, a.lamvel, a.bnd,
-                                                         a.sc);
-  return cudaGetLastError();
+  return launch_chain(g.chain, recon_sym3_kernel<EQ>, grid, dim3(L::THREADS), L::BYTES, s, umap, g, w, off, (int)zc, a.wantInd,
+                      a.F[0], a.F[1], a.F[2], a.W[0], a.W[1], a.W[2], a.src, a.status, a.lamvel, a.bnd, a.sc);
 }
 
 template <int EQ>
 static cudaError_t sym2(const ReconSymArgs &a, const CUtensorMap &umap, const Grid &g, const SymW &w, cudaStream_t s) {
   using L = Sym2<EQ>;
   const dim3 grid((unsigned)((g.nx + L::BX - 1) / L::BX), (unsigned)((g.ny + L::BY - 1) / L::BY));
-  recon_sym2_kernel<EQ><<<grid, L::THREADS, 0, s>>>(umap, g, w, a.wantInd, a.F[0], a.F[1], a.W[0], a.W[1], a.src,
-                                                  a.status, a.lamvel, a.bnd, a.sc);
-  return cudaGetLastError();
+  return launch_chain(g.chain, recon_sym2_kernel<EQ>, grid, dim3(L::THREADS), 0, s, umap, g, w, a.wantInd, a.F[0], a.F[1], a.W[0],
+                      a.W[1], a.src, a.status, a.lamvel, a.bnd, a.sc);
 }
 
 cudaError_t launch_recon_sym(int dim, int eq, const ReconSymArgs &a, const CUtensorMap &umap, const Grid &g,
