@@ -238,7 +238,7 @@ struct kfvm_solver {
   float *W[3] = {nullptr, nullptr, nullptr};  // KXRCF indicator (FP32 approximation) per own face slot and point
   uint8_t *status = nullptr;                  // 1: all linear states inside the limiter bounds
   double2 *lamvel = nullptr;                  // GLM speed maxima of each cell's linear states
-  int heavyBlocks = 0;
+  int nsm = 148;  // multiprocessors of the device
   kfvm::DevScalars *sc = nullptr;
   kfvm::DevScalars *hsc = nullptr; // pinned host copy
   RKTable rk;
@@ -606,7 +606,7 @@ int eval_front(kfvm_solver *s, int b) {
     return set_err_cuda(e, "compact");
   if ((e = run(s, KFVM_KCLASS_HEAVY, 1, [&] {
          return launch_heavy(dim, eq, s->Ub[b], s->g, s->dS, s->theta, s->F, s->src, s->heavy,
-                             s->bnd, s->sc, jd, s->heavyBlocks, st);
+                             s->bnd, s->sc, jd, s->nsm, st);
        })) != cudaSuccess)
     return set_err_cuda(e, "heavy");
   if (s->decomposed || s->hasUser) {
@@ -1001,6 +1001,7 @@ int kfvm_create(const kfvm_config *cfg, kfvm_solver **out) {
     if (cfg->nq == 2) fill_tc_weights(hS, cfg->dim, nrows);  // the tensor-core form takes 2 points only
     s->symOk = cfg->nq == 2 && cfg->eq != KFVM_EQ_SRHYDRO;
     if (!s->symOk) fill_dmma_weights(hS, nrows);
+    fill_heavy_weights(cfg->dim, cfg->eq, g, hS);
   }
   if (s->symOk && fill_sym_weights(hS.w, cfg->eq == KFVM_EQ_MHD_GLM, s->symw) != 0) {
     delete s;
@@ -1050,7 +1051,7 @@ int kfvm_create(const kfvm_config *cfg, kfvm_solver **out) {
     int dev = 0, nsm = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
-    s->heavyBlocks = (nsm > 0 ? nsm : 148) * 4; // grid-stride over the device-side count
+    if (nsm > 0) s->nsm = nsm;
   }
   {
     const int64_t nb = std::max(std::max(stage_blocks(g), errest_blocks(g.n)), forcing_blocks(g));

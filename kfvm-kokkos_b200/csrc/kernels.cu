@@ -997,8 +997,13 @@ __global__ void __launch_bounds__(256)
 template <int DIM, int EQ, int NQ = 2>
 struct HeavyShape {
   using T = Cfg<DIM, EQ, NQ>;
+  static constexpr int NVARS = T::NV;
   static constexpr int NR = LinRows<DIM, EQ, NQ>::NROWS;      // face points, then interior points
   static constexpr int NSUM = T::C + T::CC + T::NB * T::CB;   // stencil cells over all substencils
+  __host__ __device__ static constexpr int n(int s) { return s == 0 ? T::C : (s == 1 ? T::CC : T::CB); }
+  __host__ __device__ static constexpr int off(int s) {
+    return s == 0 ? 0 : (s == 1 ? T::C : T::C + T::CC + (s - 2) * T::CB);
+  }
   static constexpr int NIP = (T::NI + 1) & ~1;                // derivative rows padded to pairs
   static constexpr int NRP = (NR + 1) & ~1;                  // rows padded to pairs
   // cells per block (one thread per cell and variable); 16 where 32 cells' rows
@@ -1025,6 +1030,31 @@ struct HeavyShape {
   // derivative weights, reconstruction weights: fragments, or [s][p][row] with padded rows
   static constexpr int DER = MMA ? KS * MI * 32 : NIP * NSUM;
   static constexpr int FW = MMA ? KS * MR * 32 : NRP * NSUM;
+  static_assert(DER + FW <= kMaxHeavyW && DER % 2 == 0 && FW % 2 == 0, "weight table, copied in pairs");
+  // the table the blocks copy (DevStencil::heavy_w): derivative, then reconstruction weights
+  static void weights(const kfvm_stencil &st, double *w) {
+    for (int t = 0; t < DER + FW; t++) {
+      const bool der = t < DER;
+      const int u = der ? t : t - DER;
+      int s = 0, p, row;
+      if (MMA) {
+        const int m = der ? MI : MR, l = u % 32, mm = u / 32 % m, kst = u / (32 * m);
+        while (s + 1 < T::NSUB && kst >= ksOff(s + 1)) s++;
+        p = (kst - ksOff(s)) * 4 + (l & 3);
+        row = mm * 8 + (l >> 2);
+      } else {
+        const int len = der ? NIP : NRP;
+        while (s + 1 < T::NSUB && u >= len * off(s + 1)) s++;
+        p = (u - len * off(s)) / len;
+        row = (u - len * off(s)) % len;
+      }
+      constexpr int nfq = T::NF * T::NQF;
+      w[t] = 0.0;
+      if (p < n(s) && row < (der ? T::NI : NR))
+        w[t] = der ? st.deriv_w[s][row][p]
+                   : (row < nfq ? st.face_w[s][row / T::NQF][row % T::NQF][p] : st.cell_w[s][row - nfq][p]);
+    }
+  }
   // stencil cells of the biased substencils, in the MMA form padded by repeating the first
   static constexpr int SUB = MMA ? 4 * ks(2) : T::CB;
   static constexpr int VS = 36;                              // row stride of the stencil values [q][cell]
@@ -1037,14 +1067,12 @@ struct HeavyShape {
   static constexpr int COEF = MMA ? T::NV * T::NSUB * 32 : 0; // [v][s][cell]
   static constexpr size_t BYTES = (size_t)(DER + FW + UNION + CELLS * 2 + CELLS * T::NV + COEF) * sizeof(double) +
                                   (size_t)T::NB * SUB * sizeof(int);
-  __host__ __device__ static constexpr int n(int s) { return s == 0 ? T::C : (s == 1 ? T::CC : T::CB); }
-  __host__ __device__ static constexpr int off(int s) {
-    return s == 0 ? 0 : (s == 1 ? T::C : T::C + T::CC + (s - 2) * T::CB);
-  }
 };
 
+// (2D, five variables: four blocks per SM at 96 registers instead of two at 148 took the
+// SR four-quadrant problem at 512^2 from 0.46 to 0.32 ms per evaluation)
 template <int DIM, int EQ, int NQ>
-__global__ void __launch_bounds__(HeavyShape<DIM, EQ, NQ>::CELLS * Eos<EQ>::NV, Eos<EQ>::NV > 5 ? 1 : 2)
+__global__ void __launch_bounds__(HeavyShape<DIM, EQ, NQ>::CELLS * Eos<EQ>::NV, Eos<EQ>::NV > 5 ? 1 : (DIM == 2 ? 4 : 2))
     heavy_var_kernel(const double *__restrict__ U, Grid g, const DevStencil *__restrict__ S,
                      double *__restrict__ theta, double *__restrict__ F0, double *__restrict__ F1,
                      double *__restrict__ F2, double *__restrict__ src, const uint32_t *__restrict__ heavy,
@@ -1067,36 +1095,11 @@ __global__ void __launch_bounds__(HeavyShape<DIM, EQ, NQ>::CELLS * Eos<EQ>::NV, 
   const int tid = threadIdx.y * H::CELLS + threadIdx.x, nt = H::CELLS * NV;
   const unsigned count = sc->nheavy;
   if (blockIdx.x * H::CELLS >= count) return;  // nothing listed for this block: no weights to stage
-  if constexpr (H::MMA) {
-    for (int t = tid; t < (H::MI + H::MR) * H::KS * 32; t += nt) {
-      const bool der = t < H::DER;
-      const int u = der ? t : t - H::DER, m = der ? H::MI : H::MR, l = u % 32, mm = u / 32 % m, kst = u / (32 * m);
-      int s = 0;
-      while (s + 1 < T::NSUB && kst >= H::ksOff(s + 1)) s++;
-      const int p = (kst - H::ksOff(s)) * 4 + (l & 3), row = mm * 8 + (l >> 2);
-      double val = 0.0;
-      if (p < H::n(s)) {
-        if (der) val = row < T::NI ? st.deriv_w[s][row][p] : 0.0;
-        else val = row < NR ? st.face_w[s][row / T::NQF][row % T::NQF][p] : 0.0;  // (no interior points)
-      }
-      sDer[t] = val;
-    }
-  } else {
-    // transposed so that the rows of one stencil value are adjacent and load as
-    // 16-byte pairs
-    for (int t = tid; t < H::DER; t += nt) {
-      int s = 0;
-      while (s + 1 < T::NSUB && t >= H::NIP * H::off(s + 1)) s++;
-      const int r = t - H::NIP * H::off(s), p = r / H::NIP, i = r % H::NIP;
-      sDer[t] = i < T::NI ? st.deriv_w[s][i][p] : 0.0;
-    }
-    for (int t = tid; t < H::FW; t += nt) {
-      int s = 0;
-      while (s + 1 < T::NSUB && t >= H::NRP * H::off(s + 1)) s++;
-      const int r = t - H::NRP * H::off(s), p = r / H::NRP, row = r % H::NRP;
-      const int nfq = T::NF * T::NQF;
-      sFw[t] = row >= NR ? 0.0 : (row < nfq ? st.face_w[s][row / T::NQF][row % T::NQF][p] : st.cell_w[s][row - nfq][p]);
-    }
+  {
+    const double2 *hw = reinterpret_cast<const double2 *>(S->heavy_w);
+    double2 *sw = reinterpret_cast<double2 *>(hsm);
+#pragma unroll 8
+    for (int t = tid; t < (H::DER + H::FW) / 2; t += nt) sw[t] = hw[t];
   }
   for (int t = tid; t < T::NB * H::SUB; t += nt) {
     const int q = t % H::SUB;
@@ -1130,16 +1133,18 @@ __global__ void __launch_bounds__(HeavyShape<DIM, EQ, NQ>::CELLS * Eos<EQ>::NV, 
     };
     double *rs = sFs + x * H::CS;
     if constexpr (H::MMA) {
-      // ---- WENO-AO with both contractions on the FP64 MMA (mma.sync m8n8k4): warp v
-      // takes variable v of the block's 32 cells as the N dimension, the derivative
-      // rows (smoothness indicators) and the substencil rows (reconstructions) as M,
-      // the substencil's stencil entries as K.  Lanes of cells outside the WENO set
-      // contribute zeros and discard their results.
+      // ---- WENO-AO with both contractions on the FP64 MMA (mma.sync m8n8k4): 8 of the
+      // block's cells as the N dimension, the derivative rows (smoothness indicators)
+      // and the substencil rows (reconstructions) as M, the substencil's stencil
+      // entries as K.  Cells outside the WENO set contribute zeros and discard their
+      // results.
       const bool mine = have && (e & kHeavyWeno);
       if (__syncthreads_or(mine)) {   // uniform over the block: every warp sees the same cells
         const int lq = x & 3, ln = x >> 2;
-        double *sVw = sV + v * (T::C * H::VS);
+        double *sVw = sV + v * (T::C * H::VS);   // as thread (cell x, variable v)
         double *sCw = sCo + v * (T::NSUB * 32);
+        const double *sVt = sV + 8 * v + ln;     // as warp of the cells 8 v ..
+        double *sCt = sCo + 8 * v + 2 * lq;
         double ref[NV];
 #pragma unroll
         for (int w = 0; w < NV; w++) ref[w] = Uc[w * g.pvol];
@@ -1149,9 +1154,9 @@ __global__ void __launch_bounds__(HeavyShape<DIM, EQ, NQ>::CELLS * Eos<EQ>::NV, 
           // into the warp's [q][cell] table
           auto lin = [&](auto cTag) {
             constexpr int CV = decltype(cTag)::value;
-#pragma unroll 4
+#pragma unroll 11
             for (int q = 0; q < T::C; q++) {
-              const int64_t o = S->loff[q];
+              const int64_t o = g.loff[q];
               double u[NV];
 #pragma unroll
               for (int w = 0; w < NV; w++)
@@ -1171,56 +1176,60 @@ __global__ void __launch_bounds__(HeavyShape<DIM, EQ, NQ>::CELLS * Eos<EQ>::NV, 
             for (int q = 0; q < T::C; q++) sVw[q * H::VS + x] = 0.0;
           }
         }
-        __syncwarp();
-        // acc += W_s V_s for the fragments A of substencil s (KST steps, all loads of
-        // the unrolled steps ahead of the MMAs that use them)
-        auto contract = [&](auto kTag, int s, const double *A, double (&acc)[H::MI][4][2]) {
+        __syncthreads();
+        // Four of the warps take 8 cells each, all variables: the FP64 pipes of the SM's
+        // four partitions get equal shares (a warp per variable left two of the five
+        // on one partition), and a weight fragment feeds five MMAs instead of four.
+        // acc = W_s V_s for the fragments A of substencil s (KST steps)
+        auto contract = [&](auto kTag, int s, const double *A, double (&acc)[H::MI][H::NVARS][2]) {
           constexpr int KST = decltype(kTag)::value;
           static_assert(H::MI == H::MR, "one accumulator shape");
 #pragma unroll
           for (int mm = 0; mm < H::MI; mm++)
 #pragma unroll
-            for (int t = 0; t < 4; t++) acc[mm][t][0] = acc[mm][t][1] = 0.0;
+            for (int w = 0; w < NV; w++) acc[mm][w][0] = acc[mm][w][1] = 0.0;
           const double *As = A + H::ksOff(s) * H::MI * 32 + x;
 #pragma unroll
           for (int ksi = 0; ksi < KST; ksi++) {
             const int p = 4 * ksi + lq;
             const int q = s < 2 ? (p < (s == 0 ? T::C : T::CC) ? p : 0) : sSub[(s - 2) * H::SUB + p];
-            double bv[4], av[H::MI];
+            double bv[NV], av[H::MI];
 #pragma unroll
-            for (int t = 0; t < 4; t++) bv[t] = sVw[q * H::VS + 8 * t + ln];
+            for (int w = 0; w < NV; w++) bv[w] = sVt[(w * T::C + q) * H::VS];
 #pragma unroll
             for (int mm = 0; mm < H::MI; mm++) av[mm] = As[(ksi * H::MI + mm) * 32];
 #pragma unroll
             for (int mm = 0; mm < H::MI; mm++)
 #pragma unroll
-              for (int t = 0; t < 4; t++) dmma_884(acc[mm][t], av[mm], bv[t]);
+              for (int w = 0; w < NV; w++) dmma_884(acc[mm][w], av[mm], bv[w]);
           }
         };
-        auto substencil = [&](int s, const double *A, double (&acc)[H::MI][4][2]) {
+        auto substencil = [&](int s, const double *A, double (&acc)[H::MI][H::NVARS][2]) {
           if (s == 0) contract(std::integral_constant<int, H::ks(0)>{}, 0, A, acc);
           else if (s == 1) contract(std::integral_constant<int, H::ks(1)>{}, 1, A, acc);
           else contract(std::integral_constant<int, H::ks(2)>{}, s, A, acc);
         };
         // smoothness indicators: b = D_s V_s per substencil, beta = sum of b^2 over
-        // the rows (lane l holds rows 8 m + l / 4 of cells 8 t + 2 (l % 4) + e)
+        // the rows (lane l holds rows 8 m + l / 4 of cells 8 v + 2 (l % 4) + e)
+        if (v < 4) {
 #pragma unroll 1
-        for (int s = 0; s < T::NSUB; s++) {
-          double bd[H::MI][4][2];
-          substencil(s, sDer, bd);
+          for (int s = 0; s < T::NSUB; s++) {
+            double bd[H::MI][H::NVARS][2];
+            substencil(s, sDer, bd);
 #pragma unroll
-          for (int t = 0; t < 4; t++)
+            for (int w = 0; w < NV; w++)
 #pragma unroll
-            for (int ee = 0; ee < 2; ee++) {
-              double sq = 0.0;
+              for (int ee = 0; ee < 2; ee++) {
+                double sq = 0.0;
 #pragma unroll
-              for (int mm = 0; mm < H::MI; mm++) sq += bd[mm][t][ee] * bd[mm][t][ee];
+                for (int mm = 0; mm < H::MI; mm++) sq += bd[mm][w][ee] * bd[mm][w][ee];
 #pragma unroll
-              for (int o = 4; o < 32; o <<= 1) sq += __shfl_xor_sync(0xffffffffu, sq, o);
-              if (ln == 0) sCw[s * 32 + 8 * t + 2 * lq + ee] = sq;
-            }
+                for (int o = 4; o < 32; o <<= 1) sq += __shfl_xor_sync(0xffffffffu, sq, o);
+                if (ln == 0) sCt[(w * T::NSUB + s) * 32 + ee] = sq;
+              }
+          }
         }
-        __syncwarp();
+        __syncthreads();
         double om[T::NSUB];
 #pragma unroll
         for (int s = 0; s < T::NSUB; s++) om[s] = sCw[s * 32 + x];
@@ -1259,45 +1268,48 @@ __global__ void __launch_bounds__(HeavyShape<DIM, EQ, NQ>::CELLS * Eos<EQ>::NV, 
 #pragma unroll
           for (int s = 1; s < T::NSUB; s++) om[s] -= om[0] * gam[s];
         }
-        // each lane overwrites only its own cell's column
 #pragma unroll
         for (int s = 0; s < T::NSUB; s++) sCw[s * 32 + x] = mine ? om[s] : 0.0;
-        __syncwarp();
+        __syncthreads();
         // blend: acc = sum over s of om_s (W_s V_s), each W_s V_s summed first as the
         // reference does (per row and cell)
-        double acc[H::MR][4][2];
+        double acc[H::MR][H::NVARS][2];
+        if (v < 4) {
 #pragma unroll
-        for (int mm = 0; mm < H::MR; mm++)
+          for (int mm = 0; mm < H::MR; mm++)
 #pragma unroll
-          for (int t = 0; t < 4; t++) acc[mm][t][0] = acc[mm][t][1] = 0.0;
+            for (int w = 0; w < NV; w++) acc[mm][w][0] = acc[mm][w][1] = 0.0;
 #pragma unroll 1
-        for (int s = 0; s < T::NSUB; s++) {
-          double tt[H::MR][4][2];
-          substencil(s, sFw, tt);
+          for (int s = 0; s < T::NSUB; s++) {
+            double tt[H::MR][H::NVARS][2];
+            substencil(s, sFw, tt);
 #pragma unroll
-          for (int t = 0; t < 4; t++)
+            for (int w = 0; w < NV; w++)
 #pragma unroll
-            for (int ee = 0; ee < 2; ee++) {
-              const double c = sCw[s * 32 + 8 * t + 2 * lq + ee];
-              if (c != 0.0)
+              for (int ee = 0; ee < 2; ee++) {
+                const double c = sCt[(w * T::NSUB + s) * 32 + ee];
+                if (c != 0.0)
 #pragma unroll
-                for (int mm = 0; mm < H::MR; mm++) acc[mm][t][ee] += c * tt[mm][t][ee];
-            }
+                  for (int mm = 0; mm < H::MR; mm++) acc[mm][w][ee] += c * tt[mm][w][ee];
+              }
+          }
         }
         __syncthreads();   // every warp is done with the stencil values the rows overlay
-        const unsigned wm = __ballot_sync(0xffffffffu, mine);
-#pragma unroll
-        for (int t = 0; t < 4; t++)
+        const unsigned wm = __ballot_sync(0xffffffffu, mine);  // (of the block's cells: the same in every warp)
+        if (v < 4) {
 #pragma unroll
           for (int ee = 0; ee < 2; ee++) {
-            const int cell = 8 * t + 2 * lq + ee;
+            const int cell = 8 * v + 2 * lq + ee;
             if ((wm >> cell) & 1u)
 #pragma unroll
               for (int mm = 0; mm < H::MR; mm++) {
                 const int row = 8 * mm + ln;
-                if (row < NR) sFs[cell * H::CS + row * NV + v] = acc[mm][t][ee];
+#pragma unroll
+                for (int w = 0; w < NV; w++)
+                  if (row < NR) sFs[cell * H::CS + row * NV + w] = acc[mm][w][ee];
               }
           }
+        }
       }
     } else
     if (have && (e & kHeavyWeno)) {
@@ -2259,6 +2271,10 @@ struct Launch {
     return cudaGetLastError();
     }
   }
+  static cudaError_t heavy_weights(DevStencil &S) {
+    HeavyShape<DIM, EQ, NQ>::weights(S.w, S.heavy_w);
+    return cudaSuccess;
+  }
   static cudaError_t flag(const double *U, const Grid &g, float *const *W, double *const *F,
                           const double *theta, uint8_t *flag, DevScalars *sc, double thr, cudaStream_t s) {
     return launch_chain(g.chain, flag_kernel<DIM, EQ, NQ>, cell_grid(g), dim3(kBlockX, kBlockY), 0, s, U, g, W[0], W[1], W[2],
@@ -2272,15 +2288,20 @@ struct Launch {
   }
   static cudaError_t heavy(const double *U, const Grid &g, const DevStencil *S, double *theta,
                            double *const *F, double *src, const uint32_t *heavy, const double *bnd,
-                           DevScalars *sc, const JudgeArgs &jd, int heavy_blocks, cudaStream_t s) {
+                           DevScalars *sc, const JudgeArgs &jd, int nsm, cudaStream_t s) {
+    using H = HeavyShape<DIM, EQ, NQ>;
     // set once per process (a function-local static is initialised once, also when
     // several host threads drive solvers)
     static const cudaError_t attr = cudaFuncSetAttribute(
         heavy_var_kernel<DIM, EQ, NQ>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)HeavyShape<DIM, EQ, NQ>::BYTES);
     if (attr != cudaSuccess) return attr;
-    using H = HeavyShape<DIM, EQ, NQ>;
-    return launch_chain(g.chain, heavy_var_kernel<DIM, EQ, NQ>, dim3(heavy_blocks), dim3(H::CELLS, NV), H::BYTES, s, U, g, S,
-                        theta, F[0], F[1], F[2], src, heavy, bnd, sc, jd);
+    // The blocks stride over the list (its length is known on the device only).  The MMA
+    // form has one wave of resident blocks, which stage their weights once (Sod 97 x 75 x
+    // 51: 0.144 -> 0.116 ms per evaluation against two waves; claiming groups by an atomic
+    // instead of the stride: 0.124)
+    const int blocks = nsm * (H::MMA ? 2 : 4);
+    return launch_chain(g.chain, heavy_var_kernel<DIM, EQ, NQ>, dim3(blocks), dim3(H::CELLS, NV), H::BYTES, s, U, g,
+                        S, theta, F[0], F[1], F[2], src, heavy, bnd, sc, jd);
   }
   static cudaError_t riemann(double *const *F, double *const *G, const Grid &g, DevScalars *sc, bool same,
                              cudaStream_t s) {
@@ -2446,11 +2467,13 @@ cudaError_t launch_compact(int dim, int eq, const Grid &g, int mode, const uint8
                            const double2 *lamvel, DevScalars *sc, const JudgeArgs &jd, cudaStream_t s) {
   KFVM_DISPATCH(dim, eq, compact(g, mode, flag, wset, status, applied, theta, heavy, lamvel, sc, jd, s));
 }
+cudaError_t fill_heavy_weights(int dim, int eq, const Grid &g, DevStencil &S) {
+  KFVM_DISPATCH(dim, eq, heavy_weights(S));
+}
 cudaError_t launch_heavy(int dim, int eq, const double *U, const Grid &g, const DevStencil *S,
                          double *theta, double *const *F, double *src, const uint32_t *heavy,
-                         const double *bnd, DevScalars *sc, const JudgeArgs &jd, int heavy_blocks,
-                         cudaStream_t s) {
-  KFVM_DISPATCH(dim, eq, heavy(U, g, S, theta, F, src, heavy, bnd, sc, jd, heavy_blocks, s));
+                         const double *bnd, DevScalars *sc, const JudgeArgs &jd, int nsm, cudaStream_t s) {
+  KFVM_DISPATCH(dim, eq, heavy(U, g, S, theta, F, src, heavy, bnd, sc, jd, nsm, s));
 }
 cudaError_t launch_riemann(int dim, int eq, double *const *F, double *const *G, const Grid &g,
                            DevScalars *sc, bool same, cudaStream_t s) {

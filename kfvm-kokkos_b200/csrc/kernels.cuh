@@ -74,12 +74,16 @@ constexpr int kTcMaxK = 40, kTcMaxN = 32;
 // fragment, one double per lane): [k step][8-row tile][lane], lane -> (cell
 // 4 ks + lane % 4, row 8 nt + lane / 4), zero beyond the stencil or the rows.
 constexpr int kDmmaMaxB = 8 * 7 * 32; // 8 K-steps x 7 row tiles (54 rows)
+// and the WENO weights as the heavy pass's blocks keep them (HeavyShape::weights); the
+// largest: 3D GLM-MHD with three Gauss points
+constexpr int kMaxHeavyW = 106 * (20 + 82);
 struct DevStencil {
   kfvm_stencil w;
   int64_t loff[KFVM_MAX_CELLS];
   double lin[KFVM_MAX_CELLS * kMaxLinRows];
   alignas(16) float tcw[2][kTcMaxK * kTcMaxN];
   alignas(16) double dmma_b[kDmmaMaxB];
+  alignas(16) double heavy_w[kMaxHeavyW];
 };
 
 // The full-stencil weights for two Gauss points by parity (recon_sym.cu): the point

@@ -133,8 +133,9 @@ cudaError_t launch_compact(int dim, int eq, const Grid &g, int mode, const uint8
 // bnd: the limiter bounds (the reconstruction's, or launch_bounds' where WENO runs everywhere)
 cudaError_t launch_heavy(int dim, int eq, const double *U, const Grid &g, const DevStencil *S,
                          double *theta, double *const *F, double *src, const uint32_t *heavy,
-                         const double *bnd, DevScalars *sc, const JudgeArgs &jd, int heavy_blocks,
-                         cudaStream_t s);
+                         const double *bnd, DevScalars *sc, const JudgeArgs &jd, int nsm, cudaStream_t s);
+// host: the table of WENO weights that the heavy pass's blocks copy
+cudaError_t fill_heavy_weights(int dim, int eq, const Grid &g, DevStencil &S);
 // same: the equal-state variant of the Riemann kernels
 cudaError_t launch_riemann(int dim, int eq, double *const *F, double *const *G, const Grid &g,
                            DevScalars *sc, bool same, cudaStream_t s);
