@@ -1253,11 +1253,13 @@ __global__ void __launch_bounds__(HeavyShape<DIM, EQ, NQ>::CELLS * Eos<EQ>::NV, 
           double tot = 0.0;
 #pragma unroll
           for (int s = 0; s < T::NSUB; s++) {
-            om[s] = gam[s] / (om[s] * om[s] + 1.e-40);
+            const double b2 = om[s] * om[s];  // (a finite divisor; NaN stays)
+            om[s] = gam[s] * rcp_nr((b2 > 1e280 ? 1e280 : b2) + 1.e-40);
             tot += om[s];
           }
+          const double itot = rcp_nr(tot);
 #pragma unroll
-          for (int s = 0; s < T::NSUB; s++) om[s] /= tot;
+          for (int s = 0; s < T::NSUB; s++) om[s] *= itot;
           double dep = 0.0;
           if (sig)
 #pragma unroll
@@ -1385,11 +1387,18 @@ __global__ void __launch_bounds__(HeavyShape<DIM, EQ, NQ>::CELLS * Eos<EQ>::NV, 
       double tot = 0.0;
 #pragma unroll
       for (int s = 0; s < T::NSUB; s++) {
-        om[s] = gam[s] / (om[s] * om[s] + 1.e-40);
+        // (SR keeps the reference's quotients: the rounding of a uniform blend decides its theta)
+        const double b2 = om[s] * om[s];  // (otherwise: a finite divisor; NaN stays)
+        if constexpr (EQ == EQ_SR) om[s] = gam[s] / (b2 + 1.e-40);
+        else om[s] = gam[s] * rcp_nr((b2 > 1e280 ? 1e280 : b2) + 1.e-40);
         tot += om[s];
       }
+      const double itot = EQ == EQ_SR ? 1.0 : rcp_nr(tot);
 #pragma unroll
-      for (int s = 0; s < T::NSUB; s++) om[s] /= tot;
+      for (int s = 0; s < T::NSUB; s++) {
+        if constexpr (EQ == EQ_SR) om[s] /= tot;
+        else om[s] *= itot;
+      }
       double dep = 0.0;
       if (sig)
 #pragma unroll
@@ -2072,7 +2081,7 @@ __global__ void __launch_bounds__(128)
       double uq[NV];
 #pragma unroll
       for (int v = 0; v < NV; v++) uq[v] = Uq[v * g.pvol];
-      const double ir = 1.0 / uq[DENS];
+      const double ir = rcp_nr(uq[DENS]);
       const double pr = (g.gamma - 1.0) * (uq[ETOT] - 0.5 * (uq[MOMX] * uq[MOMX] + uq[MOMY] * uq[MOMY] +
                                                                uq[MOMZ] * uq[MOMZ]) * ir);
       vt[0][t] = uq[MOMX] * ir;
@@ -2115,7 +2124,8 @@ __global__ void __launch_bounds__(128)
         const double u = Uc[v * g.pvol];
         st[v] = u;
         hasNan = hasNan || isnan(u);
-        const double e = (u - uh) / (atol + rtol * fmax(fabs(u), fabs(uh)));
+        // (SR keeps the quotient: the last bit of the step size decides its theta in uniform gas)
+        const double tol = atol + rtol * fmax(fabs(u), fabs(uh)), e = EQ == EQ_SR ? (u - uh) / tol : (u - uh) * rcp_nr(tol);
         err += e * e;
       }
       pos = hasNan ? -1.0 : E::positivity(st);

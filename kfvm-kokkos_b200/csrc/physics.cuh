@@ -519,12 +519,13 @@ struct Eos {
 // Linearisation of the conserved variables about a reference state
 template <int EQ>
 struct VarConv {
-  double gamm, rho, irho, u, v, w, bx, by, bz, rPsi, vsq;
+  double gamm, igamm, rho, irho, u, v, w, bx, by, bz, rPsi, vsq;
   __device__ __forceinline__ VarConv(const double *ref, double gam) {
     if constexpr (EQ == EQ_SR) {
       // SRHydro_K.H:22-56: the momenta over D, linearised about (D, S) of the cell;
       // (rho, u, v, w) hold (D, Sx, Sy, Sz)
       gamm = gam - 1.0;
+      igamm = 1.0 / gamm;
       rho = ref[DENS];
       irho = 1.0 / rho;
       u = ref[MOMX];
@@ -534,11 +535,12 @@ struct VarConv {
       return;
     }
     gamm = gam - 1.0;
+    igamm = rcp_nr(gamm);
     rho = ref[DENS];
-    irho = 1.0 / rho;
-    u = ref[MOMX] / rho;
-    v = ref[MOMY] / rho;
-    w = ref[MOMZ] / rho;
+    irho = rcp_nr(rho);
+    u = ref[MOMX] * irho;
+    v = ref[MOMY] * irho;
+    w = ref[MOMZ] * irho;
     if constexpr (EQ == EQ_GLM) {
       bx = ref[MAGX];
       by = ref[MAGY];
@@ -598,10 +600,10 @@ struct VarConv {
     }
     if constexpr (EQ == EQ_GLM) {
       s[ETOT] = (vsq * s[DENS] + rho * u * s[MOMX] + rho * v * s[MOMY] + rho * w * s[MOMZ] +
-                 bx * s[MAGX] + by * s[MAGY] + bz * s[MAGZ] + s[ETOT] / gamm + rPsi * s[PSI]);
+                 bx * s[MAGX] + by * s[MAGY] + bz * s[MAGZ] + s[ETOT] * igamm + rPsi * s[PSI]);
     } else {
       s[ETOT] = (vsq * s[DENS] + rho * u * s[MOMX] + rho * v * s[MOMY] + rho * w * s[MOMZ] +
-                 s[ETOT] / gamm);
+                 s[ETOT] * igamm);
     }
     s[MOMX] = (rho * s[MOMX] + u * s[DENS]);
     s[MOMY] = (rho * s[MOMY] + v * s[DENS]);

@@ -49,16 +49,15 @@ __device__ __forceinline__ void pos_quantities(const double (&st)[Eos<EQ>::NV], 
     sm[1][t] = sr::ediff(st);
     return;
   }
-  const double ir = 1.0 / st[DENS];
+  const double ir = rcp_nr(st[DENS]);
   const double ei = E::eint_r(st, ir);
   sm[0][t] = st[DENS];
   sm[1][t] = ei;
-  sm[2][t] = sqrt(g.gamma * ((g.gamma - 1.0) * ei) * ir);
-  // velocities as the reference's divergence estimate takes them (m / rho,
-  // Common_K.H:363-378)
-  sm[3][t] = st[MOMX] / st[DENS];
-  sm[4][t] = st[MOMY] / st[DENS];
-  sm[5][t] = st[MOMZ] / st[DENS];
+  sm[2][t] = sqrt_nr(g.gamma * ((g.gamma - 1.0) * ei) * ir);
+  // velocities of the divergence estimate (Common_K.H:363-378)
+  sm[3][t] = st[MOMX] * ir;
+  sm[4][t] = st[MOMY] * ir;
+  sm[5][t] = st[MOMZ] * ir;
 }
 
 // the footprint quantities of padded cell (gi, gj, gk) into entry t of sm

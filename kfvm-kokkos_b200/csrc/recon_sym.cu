@@ -325,7 +325,7 @@ __device__ __forceinline__ void sym_cell(Ld ld, const SymW &w, const Grid &g, co
               // SpeedEstimate_K<MHD_GLM> (MHD_GLM_K.H:213-310): x components on every face
               const double asq = g.gamma * p * ir[o], absq = asq + b2[o] * ir[o], blsq = bx[o] * bx[o] * ir[o];
               const double vv = fabs(mx[o] * ir[o]);
-              const double l = sqrt(0.5 * (absq + sqrt(absq * absq - 4.0 * asq * blsq))) + vv;
+              const double l = sqrt_nr(0.5 * (absq + sqrt_nr(absq * absq - 4.0 * asq * blsq))) + vv;
               vel = vv > vel ? vv : vel;
               lam = l > lam ? l : lam;
             }
@@ -347,7 +347,7 @@ __device__ __forceinline__ void sym_foot(const double *u, int stride, double gam
   double st[NV];
 #pragma unroll
   for (int v = 0; v < NV; v++) st[v] = u[v * stride];
-  const double r = 1.0 / st[DENS], ei = Eos<EQ>::eint_r(st, r), c = gam * ((gam - 1.0) * ei) * r;
+  const double r = rcp_nr(st[DENS]), ei = Eos<EQ>::eint_r(st, r), c = gam * ((gam - 1.0) * ei) * r;
   *e = ei;
   *c2 = c >= 0.0 ? c : __longlong_as_double(0x7ff8000000000000ll);
   *ir = r;
@@ -361,8 +361,9 @@ struct SymExt {
 // and twice the velocity divergence
 template <int DIM>
 __device__ __forceinline__ void sym_bounds(const SymExt &x, double div2, SymCell<DIM> &cl) {
-  const double snd = sqrt(x.c2Min), divV = div2 / 2.0;
+  const double snd = sqrt_nr(x.c2Min), divV = div2 / 2.0;
   double kappa = 0.2;
+  // (the IEEE quotient: cold gas has snd = 0, and +-infinity decides)
   const double eta = fmin(1.0, fmax(0.0, -(kappa * snd + divV) / (kappa * snd)));
   kappa *= (1.0 - eta);
   cl.maxDens = x.rMax * (1.0 + kappa);
@@ -676,7 +677,7 @@ __global__ void __launch_bounds__(Sym3<EQ>::THREADS, Sym3<EQ>::RESIDENT)
             // SpeedEstimate_K<MHD_GLM> (MHD_GLM_K.H:213-310): x components on every face
             const double asq = g.gamma * pr * ir, absq = asq + b2 * ir, blsq = bx * bx * ir;
             const double vv = fabs(ux * ir);
-            const double l = sqrt(0.5 * (absq + sqrt(absq * absq - 4.0 * asq * blsq))) + vv;
+            const double l = sqrt_nr(0.5 * (absq + sqrt_nr(absq * absq - 4.0 * asq * blsq))) + vv;
             vel = vv > vel ? vv : vel;
             lam = l > lam ? l : lam;
           }

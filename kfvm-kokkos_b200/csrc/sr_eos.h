@@ -40,6 +40,9 @@ KFVM_SR_HD double pres_guess(double gam, const double *U) {
   return (gm2E + sqrt(gm2E * gm2E - 4.0 * gm * (U[0] * sqrt(ESsq) - ESsq))) / 2.0;
 }
 
+// |dp| / p < kRtol (a negative p stops too), without the quotient
+KFVM_SR_HD bool converged(double dp, double p) { return p > 0.0 ? fabs(dp) < kRtol * p : p < 0.0; }
+
 KFVM_SR_HD double pres_stable(double gam, const double *U, double p) {
   const double gm = gam - 1.0, gm2 = gam - 2.0, D = U[0], E = U[4], Ssq = ssq(U);
   for (int n = 0; n < kMaxIter; n++) {
@@ -47,7 +50,7 @@ KFVM_SR_HD double pres_stable(double gam, const double *U, double p) {
     const double psi = Ssq + EP * (p / gm - E) + D * rt;
     const double dpsi = (2.0 * p - gm2 * E) / gm + D * EP / rt;
     const double dp = -psi / dpsi;
-    if (fabs(dp) / p < kRtol) break;
+    if (converged(dp, p)) break;
     p += dp;
   }
   return p;
@@ -63,11 +66,14 @@ KFVM_SR_HD double pres(double gam, const double *U) {
   const double c2 = Esq * (gam * gam - 6.0 * gm) + 2.0 * Ssq * gm - Dsq * gm * gm;
   const double c3 = -2.0 * U[4] * gm2;
   for (int n = 0; n < kMaxIter; n++) {
-    if (lorenz(p, U) < 1.0 + 0.01) return pres_stable(gam, U, p);
+    // Lorentz factor 1 / sqrt(1 - S^2 / (E + p)^2) below 1.01.  The tests take no quotient or
+    // root, so an iteration has one division instead of four and a root; the iterates are the same
+    const double EP = U[4] + p;
+    if (Ssq < (1.0 - 1.0 / (1.01 * 1.01)) * (EP * EP)) return pres_stable(gam, U, p);
     const double phi = c0 + p * (c1 + p * (c2 + p * (c3 + p)));
     const double dphi = c1 + p * (2.0 * c2 + p * (3.0 * c3 + p));
     const double dp = -phi / dphi;
-    if (fabs(dp) / p < kRtol) break;
+    if (converged(dp, p)) break;
     p += dp;
   }
   return p;
