@@ -213,18 +213,26 @@ def algorithmic_bytes(cls, cfg):
         "bc_fill": 0,
     }
     if cls == "riemann":
-        return nfaces * (2 * nqf * nv * 8 + nv * 8) / d   # per launch (one direction)
+        return nfaces * (2 * nqf * nv * 8 + nv * 8)   # per launch (all directions)
     return per_cell.get(cls, 0) * n
 
 
-def algorithmic_fma(cls, cfg):
-    """FP64 fused multiply-adds per launch of the linear reconstruction contraction:
-    every (stencil cell, weight row, variable) triple once per cell."""
+def contraction_ops(cfg, direct):
+    """Operations (each one issue of the FP64 pipe) of the linear reconstruction per cell
+    and variable: every (stencil cell, weight row) pair once in the direct sum; by parity
+    the combinations of mirrored cells, then one product per combination and a butterfly
+    per group of points (a face direction, or the interior points)."""
+    d, nv, nqf, nqc, ncst, src = _shape(cfg)
+    if direct:
+        return ncst * (2 * d * nqf + (nqc if src else 0))
+    return 58 + (d + bool(src)) * 64 if d == 3 else 36 + (d + bool(src)) * 20
+
+
+def algorithmic_fma(cls, cfg, direct):
+    """Operations per launch of the linear reconstruction contraction."""
     if cls != "recon":
         return None
-    d, nv, nqf, nqc, ncst, src = _shape(cfg)
-    rows = 2 * d * nqf + (nqc if src else 0)
-    return abi.ncells(cfg) * ncst * rows * nv
+    return abi.ncells(cfg) * contraction_ops(cfg, direct) * _shape(cfg)[1]
 
 
 def load_json(path):
@@ -441,7 +449,8 @@ def run_ours(args):
     hbm = {"achieved": achieved, "peak": hbm_peak, "unit": "GB/s", "frac": achieved / hbm_peak,
            "algorithmic_bytes": algo,
            "peak_source": f"{peak_src} (MEASURED_PEAKS.json hbm_gbs)" if peaks else "fallback"}
-    fma = algorithmic_fma(dom, cfg)
+    direct = tf32_recon or cfg.eq == abi.KFVM_EQ_SRHYDRO
+    fma = algorithmic_fma(dom, cfg, direct)
     if fma is not None and tf32_recon:
         # 3xTF32 on tcgen05: three MMAs per product (hi hi, hi lo, lo hi); TF32 runs at
         # half the dense bf16 rate, so its peak is half the measured bf16 GEMM
@@ -454,11 +463,12 @@ def run_ours(args):
                                     else "half of the fallback bf16 1.59 PFLOP/s"),
                     "hbm": hbm}
     elif fma is not None:
-        # the FP64 reconstruction runs on the FP64 tensor pipe (m8n8k4 DMMA): its bound
-        # is that pipe's throughput, measured on this GPU by back-to-back MMAs
+        # the FP64 reconstruction (by parity on the FP64 units; SR's direct sum on the
+        # m8n8k4 MMA) is set against the FP64 throughput measured on this GPU by
+        # back-to-back MMAs, which the plain FP64 units share
         fp64_peak = kfvm.measure_fp64_mma()
         fp64 = 2 * fma / (avg_ms / 1e3) / 1e12
-        roofline = {"bound": "tensor", "kernel": dom, "achieved": fp64, "peak": fp64_peak, "unit": "TFLOP/s",
+        roofline = {"bound": "tensor" if direct else "fp64", "kernel": dom, "achieved": fp64, "peak": fp64_peak, "unit": "TFLOP/s",
                     "frac": fp64 / fp64_peak, "traffic": traffic, "fma_per_launch": fma, "launch_ms": avg_ms,
                     "peak_source": "measured on this GPU: FP64 m8n8k4 MMAs back to back on every SM "
                                    "(kfvm_measure_fp64_mma); FP64, so not the bf16 figure of MEASURED_PEAKS.json",
@@ -470,12 +480,11 @@ def run_ours(args):
     # the whole path: attainable zone-updates/s = min(HBM / B_zu, FP64 / F_zu)
     # B_zu: per stage U, Uprev, Utmp, Uhat in and U', Utmp, Uhat out (7 NV reals),
     #       plus the error pass (2 NV reals); F_zu: per RHS evaluation and cell the
-    #       linear contraction (2 rows C NV), d NQF Riemann solves at ~200 flops and
+    #       linear contraction (contraction_ops), d NQF Riemann solves at ~200 flops and
     #       ~300 flops of divergence / update, 4 evaluations per step (WENO cells extra)
     d_, nv_, nqf_, nqc_, ncst_, src_ = _shape(cfg)
-    rows_ = 2 * d_ * nqf_ + (nqc_ if src_ else 0)
     b_zu = 4 * 7 * nv_ * 8 + 2 * nv_ * 8
-    f_zu = 4 * (2 * rows_ * ncst_ * nv_ + d_ * nqf_ * 200 + 300)
+    f_zu = 4 * (2 * contraction_ops(cfg, direct) * nv_ + d_ * nqf_ * 200 + 300)
     fp64_peak_ = (roofline["peak"] * 1e12 if roofline["unit"] == "TFLOP/s" and not tf32_recon
                   else kfvm.measure_fp64_mma() * 1e12)
     att_hbm, att_fp64 = hbm_peak * 1e9 / b_zu, fp64_peak_ / f_zu

@@ -97,8 +97,9 @@ constexpr uint32_t kHeavyJudgeOnly = 0x20000000u; // judged but outside the WENO
                                                   // says troubled (the cell-level fallback)
 constexpr uint32_t kHeavyCell = kHeavyCellMax;
 
-// Linear reconstruction of every cell on the FP64 tensor cores (mma.sync m8n8k4,
-// the FP64 MMA of sm_100a; tcgen05 has no FP64 kind).  Per warp: one row of 32 cells
+// Linear reconstruction by the direct sum (three Gauss points, and SR; recon_sym.cu has the
+// rest) on the FP64 tensor cores (mma.sync m8n8k4, the FP64 MMA of sm_100a; tcgen05 has no
+// FP64 kind).  Per warp: one row of 32 cells
 // of the block, in 4 groups of 8 cells.  For one group and variable v,
 //   D[cell][row] = sum_k A[cell][k] B[k][row],  A = U(cell + offset k), B = weights,
 // K runs over the stencil in steps of 4, N over the weight rows in tiles of 8;
