@@ -445,7 +445,7 @@ def run_ours(args):
     case = f"{cfg.dim}d_{('hydro', 'ns', 'glm', 'sr')[cfg.eq]}"
     per_cell = traffic_tbl.get("cases", {}).get(case, {}).get("bytes_per_cell", {}).get(
         "recon_tc" if args.precision == "tf32x3" and dom == "recon" else dom)
-    traffic = per_cell * n if per_cell is not None else None
+    traffic = per_cell * n * (cfg.dim if dom == "riemann" else 1) if per_cell is not None else None
     hbm = {"achieved": achieved, "peak": hbm_peak, "unit": "GB/s", "frac": achieved / hbm_peak,
            "algorithmic_bytes": algo,
            "peak_source": f"{peak_src} (MEASURED_PEAKS.json hbm_gbs)" if peaks else "fallback"}

@@ -79,7 +79,8 @@ __global__ void __launch_bounds__(256)
 
 // ---------------------------------------------------------------------------
 // Stage front end, four kernels:
-//   recon    linear face states of every cell (FP64 MMA) written to the face
+//   recon    linear face states of every cell (by parity: recon_sym.cu, or the
+//            direct sum on the FP64 MMA) written to the face
 //            arrays, the KXRCF indicator p/rho^gamma (FP32 approximation) at each
 //            own face point written to W, and whether every state lies strictly
 //            inside the positivity limiter's bounds (then theta = 1 exactly as in
