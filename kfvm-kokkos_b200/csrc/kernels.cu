@@ -30,7 +30,7 @@ __device__ __forceinline__ int64_t axis_map(int64_t i, int64_t n, int bcLo, int 
 // 64-bit divisions took longer than the copies (8 -> 4 us at 32^2).
 template <int DIM, int NV>
 __global__ void __launch_bounds__(256)
-    bc_fill_kernel(double *__restrict__ U, const __grid_constant__ Grid g, DevScalars *__restrict__ sc) {
+    bc_fill_kernel(double *U, const __grid_constant__ Grid g, DevScalars *sc) {
   pdl_begin();
   if (sc && blockIdx.x == 0 && threadIdx.x == 0) {
     sc->glm_lam_bits = sc->glm_vel_bits = 0ull;
@@ -70,11 +70,11 @@ __global__ void __launch_bounds__(256)
   unsigned flip = (i < 0 ? g.bflip[0] : (i >= g.nx ? g.bflip[1] : 0u)) ^
                   (j < 0 ? g.bflip[2] : (j >= g.ny ? g.bflip[3] : 0u));
   if (DIM == 3) flip ^= k < 0 ? g.bflip[4] : (k >= g.nz ? g.bflip[5] : 0u);
+  double x[NV];  // (every load before the stores, which may alias them)
 #pragma unroll
-  for (int v = 0; v < NV; v++) {
-    const double x = U[v * g.pvol + src];
-    U[v * g.pvol + dst] = (flip >> v) & 1u ? -x : x;
-  }
+  for (int v = 0; v < NV; v++) x[v] = U[v * g.pvol + src];
+#pragma unroll
+  for (int v = 0; v < NV; v++) U[v * g.pvol + dst] = (flip >> v) & 1u ? -x[v] : x[v];
 }
 
 // ---------------------------------------------------------------------------
@@ -384,7 +384,7 @@ __global__ void __launch_bounds__(DmmaTile<DIM>::THREADS, (DIM == 2 && NQ == 2 &
                      double *__restrict__ F0, double *__restrict__ F1, double *__restrict__ F2,
                      float *__restrict__ W0, float *__restrict__ W1, float *__restrict__ W2,
                      double *__restrict__ src, uint8_t *__restrict__ status, double2 *__restrict__ lamvel,
-                     double *__restrict__ bnd, DevScalars *__restrict__ sc) {
+                     double *__restrict__ bnd, DevScalars *sc) {
   using T = Cfg<DIM, EQ, NQ>;
   using Sh = DmmaShape<DIM, EQ, NQ>;
   using D = DmmaTile<DIM>;
@@ -817,11 +817,11 @@ __device__ __forceinline__ void kxrcf_face(const Grid &g, int fc, int64_t i, int
 
 template <int DIM, int EQ, int NQ>
 __global__ void __launch_bounds__(128, 8)
-    flag_kernel(const double *__restrict__ U, Grid g, const float *__restrict__ W0,
-                const float *__restrict__ W1, const float *__restrict__ W2,
-                const double *__restrict__ F0, const double *__restrict__ F1,
-                const double *__restrict__ F2, const double *__restrict__ theta,
-                uint8_t *__restrict__ flag, DevScalars *__restrict__ sc, double wThresh) {
+    flag_kernel(const double *U, Grid g, const float *W0,
+                const float *W1, const float *W2,
+                const double *F0, const double *F1,
+                const double *F2, const double *theta,
+                uint8_t *__restrict__ flag, DevScalars *sc, double wThresh) {
   pdl_begin();
   using T = Cfg<DIM, EQ, NQ>;
   constexpr int NV = T::NV;
@@ -926,10 +926,10 @@ __global__ void __launch_bounds__(128, 8)
 // theta = 1 for in-bounds linear cells, and the heavy list.
 template <int DIM, int EQ>
 __global__ void __launch_bounds__(256)
-    compact_kernel(Grid g, int mode, const uint8_t *__restrict__ flag, uint8_t *__restrict__ wset,
-                   const uint8_t *__restrict__ status, uint8_t *__restrict__ applied,
+    compact_kernel(Grid g, int mode, const uint8_t *flag, uint8_t *wset,
+                   const uint8_t *status, uint8_t *__restrict__ applied,
                    double *__restrict__ theta, uint32_t *__restrict__ heavy,
-                   const double2 *__restrict__ lamvel, DevScalars *__restrict__ sc, JudgeArgs jd) {
+                   const double2 *lamvel, DevScalars *sc, JudgeArgs jd) {
   pdl_begin();
   const int64_t c = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   bool useWeno = false, push = false, judged = false, judgeOnly = false;
@@ -1075,10 +1075,10 @@ struct HeavyShape {
 // SR four-quadrant problem at 512^2 from 0.46 to 0.32 ms per evaluation)
 template <int DIM, int EQ, int NQ>
 __global__ void __launch_bounds__(HeavyShape<DIM, EQ, NQ>::CELLS * Eos<EQ>::NV, Eos<EQ>::NV > 5 ? 1 : (DIM == 2 ? 4 : 2))
-    heavy_var_kernel(const double *__restrict__ U, Grid g, const DevStencil *__restrict__ S,
-                     double *__restrict__ theta, double *__restrict__ F0, double *__restrict__ F1,
-                     double *__restrict__ F2, double *__restrict__ src, const uint32_t *__restrict__ heavy,
-                     const double *__restrict__ bnd, DevScalars *__restrict__ sc, JudgeArgs jd) {
+    heavy_var_kernel(const double *U, Grid g, const DevStencil *__restrict__ S,
+                     double *__restrict__ theta, double *F0, double *F1,
+                     double *F2, double *src, const uint32_t *heavy,
+                     const double *bnd, DevScalars *sc, JudgeArgs jd) {
   pdl_begin();
   using T = Cfg<DIM, EQ, NQ>;
   using H = HeavyShape<DIM, EQ, NQ>;
@@ -1625,8 +1625,8 @@ struct RiemannShape {
 };
 
 template <int DIM, int EQ, int D, int NQ, bool SAME>
-__device__ __forceinline__ void riemann_dir(const double *__restrict__ F, double *__restrict__ G, const Grid &g,
-                                            uint64_t fdiv, DevScalars *__restrict__ sc,
+__device__ __forceinline__ void riemann_dir(const double *F, double *__restrict__ G, const Grid &g,
+                                            uint64_t fdiv, DevScalars *sc,
                                             double (*part)[Cfg<DIM, EQ, NQ>::NQF][Eos<EQ>::NV][32], unsigned *cnt) {
   using T = Cfg<DIM, EQ, NQ>;
   using E = Eos<EQ>;
@@ -1675,8 +1675,8 @@ __device__ __forceinline__ void riemann_dir(const double *__restrict__ F, double
     double uL[NV], uR[NV], Fq[NV];
 #pragma unroll
     for (int v = 0; v < NV; v++) {
-      uL[v] = __ldg(pL);
-      uR[v] = __ldg(pR);
+      uL[v] = *pL;
+      uR[v] = *pR;
       pL += nf;
       pR += nf;
     }
@@ -1743,7 +1743,7 @@ struct RiemannArgs {
 
 template <int DIM, int EQ, int NQ, bool SAME>
 __global__ void __launch_bounds__(RiemannShape<DIM, EQ, NQ>::THREADS, RiemannShape<DIM, EQ, NQ>::RESIDENT)
-    riemann_kernel(const __grid_constant__ RiemannArgs a, const __grid_constant__ Grid g, DevScalars *__restrict__ sc) {
+    riemann_kernel(const __grid_constant__ RiemannArgs a, const __grid_constant__ Grid g, DevScalars *sc) {
   pdl_begin();
   using R = RiemannShape<DIM, EQ, NQ>;
   __shared__ double part[R::ROWS][R::NQF][Eos<EQ>::NV][32];
@@ -1763,10 +1763,10 @@ __global__ void __launch_bounds__(RiemannShape<DIM, EQ, NQ>::THREADS, RiemannSha
 // summed over the points before they meet div B, which is the same for all of them
 // (per value before: stage kernel 0.29 ms at 1024^2 and 0.47 ms at 96^3; now 0.175 and 0.26 ms).
 template <int DIM, int NQ>
-__device__ __forceinline__ void glm_sources(const double *__restrict__ Uc, const Grid &g, int64_t i, int64_t j,
-                                            int64_t k, int64_t c, const double *__restrict__ F0,
-                                            const double *__restrict__ F1, const double *__restrict__ F2,
-                                            const double *__restrict__ src, double th, double *rhs) {
+__device__ __forceinline__ void glm_sources(const double *Uc, const Grid &g, int64_t i, int64_t j,
+                                            int64_t k, int64_t c, const double *F0,
+                                            const double *F1, const double *F2,
+                                            const double *src, double th, double *rhs) {
   using T = Cfg<DIM, EQ_GLM, NQ>;
   constexpr int NV = 9, NQF = T::NQF;
   constexpr int nzq = DIM == 3 ? NQ : 1;
@@ -2030,13 +2030,13 @@ __device__ void viscous(const double (*vt)[PosTile<DIM>::N], const Grid &g, int 
 // flux divergence (+ viscous, + GLM sources) fused with the RK register update
 template <int DIM, int EQ, int NQ>
 __global__ void __launch_bounds__(128)
-    stage_kernel(const double *__restrict__ U, double *__restrict__ Unext,
-                 const double *__restrict__ Uprev, double *__restrict__ Uhat,
-                 double *__restrict__ Utmp, double *__restrict__ K, Grid g,
-                 const double *__restrict__ G0, const double *__restrict__ G1,
-                 const double *__restrict__ G2, const double *__restrict__ F0,
-                 const double *__restrict__ F1, const double *__restrict__ F2,
-                 const double *__restrict__ src, const double *__restrict__ theta, int mode,
+    stage_kernel(const double *U, double *__restrict__ Unext,
+                 const double *Uprev, double *Uhat,
+                 double *Utmp, double *__restrict__ K, Grid g,
+                 const double *G0, const double *G1,
+                 const double *G2, const double *F0,
+                 const double *F1, const double *F2,
+                 const double *src, const double *theta, int mode,
                  StageCoef co, double Re, double Pr, double atol, double rtol,
                  double *__restrict__ part) {
   pdl_begin();
@@ -2101,30 +2101,43 @@ __global__ void __launch_bounds__(128)
 #pragma unroll
       for (int v = 0; v < NV; v++) K[v * g.n + c] = r[v];
     } else if (mode == STAGE_UPDATE) {
+      // every load before the stores, which may alias them (the registers this takes, 72 instead
+      // of 40 for Euler, cost nothing: per launch Sod 256^3 0.64 -> 0.56 ms, Navier-Stokes
+      // 160^3 0.30 -> 0.24)
+      double u[NV], uh[NV], ut[NV], up[NV];
 #pragma unroll
       for (int v = 0; v < NV; v++) {
-        const double u = Uc[v * g.pvol];
-        double un = co.g1 * u;
+        u[v] = Uc[v * g.pvol];
+        uh[v] = Uhat[v * g.n + c];
+        ut[v] = co.use_tmp ? Utmp[v * g.n + c] : 0.0;
+        up[v] = co.g3 != 0.0 ? Uprev[v * g.pvol + p] : 0.0;
+      }
+#pragma unroll
+      for (int v = 0; v < NV; v++) {
+        double un = co.g1 * u[v];
         if (co.use_tmp) {
-          const double ut = Utmp[v * g.n + c] + co.delta * u;
-          Utmp[v * g.n + c] = ut;
-          un += co.g2 * ut;
+          ut[v] += co.delta * u[v];
+          Utmp[v * g.n + c] = ut[v];
+          un += co.g2 * ut[v];
         }
-        if (co.g3 != 0.0) un += co.g3 * Uprev[v * g.pvol + p];
+        if (co.g3 != 0.0) un += co.g3 * up[v];
         un += co.betaDt * r[v];
         Unext[v * g.pvol + p] = un;
-        Uhat[v * g.n + c] += co.bhatDt * r[v];
+        Uhat[v * g.n + c] = uh[v] + co.bhatDt * r[v];
       }
     } else { // STAGE_FSAL: K = rhs, Uhat += bhat_fsal dt K, error estimate
       bool hasNan = false;
-      double st[NV];
+      double st[NV], uha[NV];
+#pragma unroll
+      for (int v = 0; v < NV; v++) {
+        st[v] = Uc[v * g.pvol];
+        uha[v] = Uhat[v * g.n + c];
+      }
 #pragma unroll
       for (int v = 0; v < NV; v++) {
         K[v * g.n + c] = r[v];
-        const double uh = Uhat[v * g.n + c] + co.bhatDt * r[v];
+        const double uh = uha[v] + co.bhatDt * r[v], u = st[v];
         Uhat[v * g.n + c] = uh;
-        const double u = Uc[v * g.pvol];
-        st[v] = u;
         hasNan = hasNan || isnan(u);
         // (SR keeps the quotient: the last bit of the step size decides its theta in uniform gas)
         const double tol = atol + rtol * fmax(fabs(u), fabs(uh)), e = EQ == EQ_SR ? (u - uh) / tol : (u - uh) * rcp_nr(tol);
@@ -2161,7 +2174,7 @@ __global__ void __launch_bounds__(128)
 }
 
 // fixed-order sum of the block partials (one block)
-__global__ void __launch_bounds__(1024) finalize_kernel(const double *__restrict__ part,
+__global__ void __launch_bounds__(1024) finalize_kernel(const double *part,
                                                          int64_t nblk, DevScalars *sc) {
   pdl_begin();
   __shared__ double se[1024], sp[1024];
@@ -2189,9 +2202,9 @@ __global__ void __launch_bounds__(1024) finalize_kernel(const double *__restrict
 // first stage of a step (RKFSAL_StagePre_K, Numeric_K.H:198-220)
 template <int NV>
 __global__ void __launch_bounds__(128)
-    stage_pre_kernel(double *__restrict__ U1, const double *__restrict__ Uprev,
+    stage_pre_kernel(double *__restrict__ U1, const double *Uprev,
                      double *__restrict__ Uhat, double *__restrict__ Utmp,
-                     const double *__restrict__ K, Grid g, double betaDt, double bhatDt,
+                     const double *K, Grid g, double betaDt, double bhatDt,
                      int use_tmp) {
   pdl_begin();
   const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;

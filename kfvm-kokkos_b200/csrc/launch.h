@@ -33,6 +33,13 @@ struct StageArgs {
 // short kernels overlaps their run.  Every kernel launched this way has to call
 // pdl_begin(); other work on the stream is ordered as usual.
 //
+// Such a kernel exists while its predecessor still writes, so what it reads of the
+// predecessors' arrays is not constant over its life, which the non-coherent load path
+// (ld.global.nc: __ldg, or const __restrict__) presumes; and a load through any
+// __restrict__ pointer may be moved above the wait, whose memory clobber does not reach an
+// array that nothing else is said to name.  So in these kernels only tables written at
+// creation (DevStencil) and arrays that the kernel itself only writes are __restrict__.
+//
 // early: Grid::chain, which is set in 2D and up to 2^16 cells in 3D.  Whole passes with
 // and without: Euler 2D 32^2 0.58 and 0.83 ms, 1024^2 12.9 and 13.3, 2048^2 26.0 and 26.3;
 // Euler 3D 40^3 4.50 and 4.65, but 50^3 5.18 and 4.99, 256^3 245 and 232: the 3D kernels

@@ -427,7 +427,7 @@ __global__ void __launch_bounds__(Sym3<EQ>::THREADS, Sym3<EQ>::RESIDENT)
                       double *__restrict__ F0, double *__restrict__ F1, double *__restrict__ F2,
                       float *__restrict__ W0, float *__restrict__ W1, float *__restrict__ W2,
                       double *__restrict__ src, uint8_t *__restrict__ status, double2 *__restrict__ lamvel,
-                      double *__restrict__ bnd, DevScalars *__restrict__ sc) {
+                      double *__restrict__ bnd, DevScalars *sc) {
   pdl_begin();
   using L = Sym3<EQ>;
   using E = Eos<EQ>;
@@ -716,7 +716,7 @@ __global__ void __launch_bounds__(Sym2<EQ>::THREADS, Sym2<EQ>::RESIDENT)
                       const __grid_constant__ SymW w, int wantInd, double *__restrict__ F0, double *__restrict__ F1,
                       float *__restrict__ W0, float *__restrict__ W1, double *__restrict__ src,
                       uint8_t *__restrict__ status, double2 *__restrict__ lamvel, double *__restrict__ bnd,
-                      DevScalars *__restrict__ sc) {
+                      DevScalars *sc) {
   pdl_begin();
   using L = Sym2<EQ>;
   constexpr int NV = L::NV, TX = L::TX, TN = L::TN, PX = L::PX, PN = L::PN;
