@@ -286,6 +286,19 @@ int kfvm_selftest_wait(double limit_s, int32_t *gave_up, double *waited_s);
  * x * rcp(y) and x / y.  No reference counterpart (the reference divides). */
 int kfvm_selftest_rcp(int64_t n, uint64_t seed, int64_t *max_ulp, double *max_rel_quot);
 
+/* Self-tests of the device arithmetic on the caller's values (host arrays; no reference
+ * counterpart).  kfvm_selftest_math evaluates one function at n points, in = [3][n]:
+ *   KFVM_SELFTEST_SQRT           the square root of in[0]
+ *   KFVM_SELFTEST_ONE_MINUS_POW  1 - (in[0] / in[1])^in[2], the HLLC shear factor
+ *   KFVM_SELFTEST_POWER          in[1]^-in[0], the 2D indicator's power (NaN: not covered)
+ * kfvm_selftest_flux solves n Riemann problems of an equation system in direction dir:
+ * in = [uL, uR][NV][n], out = the flux [NV][n], then the largest wave speed [n]; ch is the
+ * cleaning speed of GLM-MHD. */
+enum { KFVM_SELFTEST_SQRT = 0, KFVM_SELFTEST_ONE_MINUS_POW = 1, KFVM_SELFTEST_POWER = 2 };
+int kfvm_selftest_math(int32_t fn, int64_t n, const double *in, double *out);
+int kfvm_selftest_flux(int32_t eq, int32_t rs, double gamma, double ch, int32_t dir, int64_t n, const double *in,
+                       double *out);
+
 /* ---- Learned troubled-cell indicator (KFVM_IND_MLP) -----------------------
  * No reference counterpart: it replaces the KXRCF selector (WenoSelect_K,
  * src/numeric/Numeric_K.H:292-398) with a 2x32 MLP over the normalised 5^d

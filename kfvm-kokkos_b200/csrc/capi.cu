@@ -10,6 +10,7 @@
 #include <cmath>
 #include <cstdio>
 #include <cstring>
+#include <functional>
 #include <random>
 #include <algorithm>
 #include <map>
@@ -1593,6 +1594,38 @@ int kfvm_selftest_rcp(int64_t n, uint64_t seed, int64_t *max_ulp, double *max_re
   std::memcpy(&q, &h[1], sizeof(q));
   *max_rel_quot = q;
   return KFVM_OK;
+}
+
+// in (host) to the device, a probe, out back
+static int selftest_arrays(size_t nIn, const double *in, size_t nOut, double *out, const char *what,
+                           const std::function<cudaError_t(const double *, double *)> &probe) {
+  double *d = nullptr;
+  cudaError_t e = cudaMalloc((void **)&d, (nIn + nOut) * sizeof(double));
+  if (e == cudaSuccess) e = cudaMemcpy(d, in, nIn * sizeof(double), cudaMemcpyHostToDevice);
+  if (e == cudaSuccess) e = probe(d, d + nIn);
+  if (e == cudaSuccess) e = cudaMemcpy(out, d + nIn, nOut * sizeof(double), cudaMemcpyDeviceToHost);
+  cudaFree(d);
+  return e == cudaSuccess ? KFVM_OK : set_err_cuda(e, what);
+}
+
+int kfvm_selftest_math(int32_t fn, int64_t n, const double *in, double *out) {
+  if (fn < KFVM_SELFTEST_SQRT || fn > KFVM_SELFTEST_POWER || n <= 0 || n > ((int64_t)1 << 28) || !in || !out)
+    return fail(KFVM_ERR_ARG, "bad argument");
+  return selftest_arrays(3 * (size_t)n, in, (size_t)n, out, "math probe",
+                         [&](const double *i, double *o) { return kfvm::launch_math_probe(fn, n, i, o, 0); });
+}
+
+int kfvm_selftest_flux(int32_t eq, int32_t rs, double gamma, double ch, int32_t dir, int64_t n, const double *in,
+                       double *out) {
+  if (eq < KFVM_EQ_HYDRO || eq > KFVM_EQ_SRHYDRO || rs < 0 || rs > 2 || dir < 0 || dir > 2 || n <= 0 ||
+      n > ((int64_t)1 << 28) || !in || !out)
+    return fail(KFVM_ERR_ARG, "bad argument");
+  if (rs == KFVM_RS_HLLC && (eq == KFVM_EQ_MHD_GLM || eq == KFVM_EQ_SRHYDRO))
+    return fail(KFVM_ERR_ARG, "HLLC is for Euler and Navier-Stokes");
+  const size_t nv = eq == KFVM_EQ_MHD_GLM ? 9 : 5;
+  return selftest_arrays(2 * nv * n, in, (nv + 1) * n, out, "flux probe", [&](const double *i, double *o) {
+    return kfvm::launch_flux_probe(eq, rs, gamma, ch, dir, n, i, o, 0);
+  });
 }
 
 int kfvm_get_faces(kfvm_solver *s, int32_t dir, double *out) {

@@ -98,7 +98,8 @@ __device__ __forceinline__ double one_minus_pow(double pMin, double pMax, double
     r = fma(t, r, 1.0);
     return -(t * r);
   }
-  return 1.0 - exp(M * log(fmin(1.0, pMin * rcp_nr(pMax))));
+  // (equal pressures that the series does not cover: both zero, where M is NaN)
+  return pMin == pMax ? 0.0 : 1.0 - exp(M * log(fmin(1.0, pMin * rcp_nr(pMax))));
 }
 
 template <int EQ>

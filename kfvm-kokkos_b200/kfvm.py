@@ -53,6 +53,8 @@ def lib():
         L.kfvm_set_precision.argtypes = [P, I32]
         L.kfvm_selftest_wait.argtypes = [D, C.POINTER(I32), C.POINTER(D)]
         L.kfvm_selftest_rcp.argtypes = [I64, C.c_uint64, C.POINTER(I64), C.POINTER(D)]
+        L.kfvm_selftest_math.argtypes = [I32, I64, P, P]
+        L.kfvm_selftest_flux.argtypes = [I32, I32, D, D, I32, I64, P, P]
         L.kfvm_mlp_num_weights.argtypes = [I32]
         L.kfvm_mlp_init_weights.argtypes = [P, C.c_uint64]
         L.kfvm_mlp_set_weights.argtypes = [P, P, I64]
@@ -127,6 +129,28 @@ def selftest_rcp(n=1 << 24, seed=5):
     u, q = C.c_int64(), C.c_double()
     _check(lib().kfvm_selftest_rcp(int(n), int(seed), C.byref(u), C.byref(q)), "kfvm_selftest_rcp")
     return u.value, q.value
+
+
+SELFTEST_SQRT, SELFTEST_ONE_MINUS_POW, SELFTEST_POWER = 0, 1, 2
+
+
+def selftest_math(fn, *args):
+    """kfvm_selftest_math: the device function fn at the points of up to three arrays."""
+    a = np.zeros((3, len(args[0])))
+    a[:len(args)] = args
+    out = np.empty(a.shape[1])
+    _check(lib().kfvm_selftest_math(int(fn), a.shape[1], a.ctypes.data, out.ctypes.data), "kfvm_selftest_math")
+    return out
+
+
+def selftest_flux(eq, rs, gamma, u_left, u_right, dir=0, ch=0.0):
+    """kfvm_selftest_flux: (flux [nv][n], largest wave speed [n]) of n Riemann problems."""
+    a = np.ascontiguousarray(np.stack([u_left, u_right]), dtype=np.float64)
+    nv, n = a.shape[1:]
+    out = np.empty((nv + 1, n))
+    _check(lib().kfvm_selftest_flux(int(eq), int(rs), float(gamma), float(ch), int(dir), n, a.ctypes.data,
+                                    out.ctypes.data), "kfvm_selftest_flux")
+    return out[:nv], out[nv]
 
 
 def forcing_num_modes(dim):
