@@ -40,8 +40,9 @@ KFVM_SR_HD double pres_guess(double gam, const double *U) {
   return (gm2E + sqrt(gm2E * gm2E - 4.0 * gm * (U[0] * sqrt(ESsq) - ESsq))) / 2.0;
 }
 
-// |dp| / p < kRtol (a negative p stops too), without the quotient
-KFVM_SR_HD bool converged(double dp, double p) { return p > 0.0 ? fabs(dp) < kRtol * p : p < 0.0; }
+// |dp| / p < kRtol without the quotient: a negative p stops too, a dp that is not a number
+// never does (p then takes it, and the recovery has visibly failed)
+KFVM_SR_HD bool converged(double dp, double p) { return p > 0.0 ? fabs(dp) < kRtol * p : p < 0.0 && dp == dp; }
 
 KFVM_SR_HD double pres_stable(double gam, const double *U, double p) {
   const double gm = gam - 1.0, gm2 = gam - 2.0, D = U[0], E = U[4], Ssq = ssq(U);
