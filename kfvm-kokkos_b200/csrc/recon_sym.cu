@@ -544,6 +544,7 @@ __global__ void __launch_bounds__(Sym3<EQ>::THREADS, Sym3<EQ>::RESIDENT)
       qo = sym_plane<TX>(u + 2 * L::PLANE, c0);
     }
   }
+  smem_release_to_copies();  // (the column's values above are used much later)
   __syncthreads();
   if (L::KEEP && ok && tid == 0) issue(k0 + 2);  // into the slot of plane k0 - 2
   if (ok) fill_foot(p0 + 2 * L::PLANE, 0);
@@ -583,6 +584,7 @@ __global__ void __launch_bounds__(Sym3<EQ>::THREADS, Sym3<EQ>::RESIDENT)
     const int par = (k - k0) & 1;
     ok = ok && wait(k + 2);
     if (ok && k + 1 < k1) fill_foot(ring + sq, 1 - par);
+    smem_release_to_copies();
     if (!__syncthreads_and(ok)) {
       // a plane never arrived: record it, give the copies in flight a bounded time
       // to land, and leave

@@ -31,6 +31,13 @@ __device__ __forceinline__ void tma_prefetch_map(const CUtensorMap *map) {
   asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(map)) : "memory");
 }
 
+// Orders this thread's ordinary accesses to shared memory before copies into it that are
+// issued behind the next barrier.  A barrier alone does not: a load whose value is not
+// needed yet may still wait in the load/store queue when the copy lands.
+__device__ __forceinline__ void smem_release_to_copies() {
+  asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+}
+
 // untiled bulk copy of `bytes` (a multiple of 16; both addresses 16-byte aligned)
 __device__ __forceinline__ void bulk_load(uint32_t dst, const void *src, uint32_t bytes, uint32_t bar) {
   asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst),
