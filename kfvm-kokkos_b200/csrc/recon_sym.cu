@@ -41,6 +41,7 @@
 
 #include "kernels.cuh"
 #include "launch.h"
+#include "plane_ring.h"
 #include "recon_common.cuh"
 #include "tma.cuh"
 
@@ -445,21 +446,18 @@ __global__ void __launch_bounds__(Sym3<EQ>::THREADS, Sym3<EQ>::RESIDENT)
   unsigned *mask = reinterpret_cast<unsigned *>(smem + L::OFF_M);
   const int i0 = (int)(blockIdx.x * L::BX), j = (int)blockIdx.y;
   const int k0 = (int)blockIdx.z * zc, k1 = k0 + zc < (int)g.nz ? k0 + zc : (int)g.nz;
-  // plane p (k0 - 2 .. k1 + 1) is load p - k0 + 2: slot and barrier that modulo RING
+  using Ring = PlaneRing<L::RING>;
   const int last = k1 + 1;
   auto issue = [&](int p) {
-    const int n = p - k0 + 2, s = n % L::RING;
+    const int s = Ring::slot(k0, p);
     mbar_arrive_expect_tx(bar + 8 * s, (uint32_t)(NV * TN * 8));
     tma_load_4d(smem_u32(ring + s * L::PLANE), &umap, i0, j, p + kRad, 0, bar + 8 * s);
   };
-  auto wait = [&](int p) {
-    const int n = p - k0 + 2;
-    return mbar_wait(bar + 8 * (n % L::RING), (uint32_t)(n / L::RING) & 1u);
-  };
+  auto wait = [&](int p) { return mbar_wait(bar + 8 * Ring::slot(k0, p), Ring::parity(k0, p)); };
   if (tid == 0) {
     for (int s = 0; s < L::RING; s++) mbar_init(bar + 8 * s, 1);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-    for (int p = k0 - 2; p < k0 - 2 + L::RING && p <= last; p++) issue(p);
+    for (int p = k0 - 2; p <= Ring::started(k0, last); p++) issue(p);
   }
   __syncthreads();
   const int own = 2 * TX + lane + 2, pown = PX + lane + 1;
@@ -590,7 +588,7 @@ __global__ void __launch_bounds__(Sym3<EQ>::THREADS, Sym3<EQ>::RESIDENT)
       // to land, and leave
       if (tid == 0) {
         atomicExch(&sc->fault, 1u);
-        for (int p = k; p <= k + 2 && p <= last; p++) wait(p);
+        for (int p = Ring::flying_from(k0, k); p <= Ring::flying_to(k, last); p++) wait(p);
       }
       return;
     }
