@@ -422,9 +422,10 @@ __global__ void __launch_bounds__(DmmaTile<DIM>::THREADS, (DIM == 2 && NQ == 2 &
   }
   __syncthreads();  // the barrier's initialisation is visible to every waiting thread
   if (!mbar_wait(bar, 0)) {
-    // the tile never arrived: record it, give the copies in flight a bounded time
-    // to land, and leave
-    if (tid == 0) atomicExch(&sc->fault, 1u);
+    // the tile never arrived: record it (each thread for itself: its cells stay
+    // unwritten, whatever the others saw), give the copies in flight a bounded time to
+    // land, and leave
+    atomicExch(&sc->fault, 1u);
     mbar_wait(bar, 0);
     return;
   }

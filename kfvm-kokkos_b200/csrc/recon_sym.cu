@@ -734,7 +734,8 @@ __global__ void __launch_bounds__(Sym2<EQ>::THREADS, Sym2<EQ>::RESIDENT)
   }
   __syncthreads();
   if (!mbar_wait(bar, 0)) {
-    if (tid == 0) atomicExch(&sc->fault, 1u);
+    // (each thread for itself: its cell stays unwritten, whatever the others saw)
+    atomicExch(&sc->fault, 1u);
     mbar_wait(bar, 0);  // a bounded time for the copy to land
     return;
   }

@@ -39,3 +39,14 @@ def test_refills_follow_a_fence_and_a_barrier(src, start, refill):
         fences = [k for k, x in enumerate(span) if re.match(FENCE, x)]
         assert bars and fences and min(fences) < max(bars), (src, span)
     assert found
+
+
+@pytest.mark.parametrize("src", ["kernels.cu", "recon_sym.cu", "recon_tc.cu", "mlp.cu"])
+def test_whoever_gives_up_records_it(src):
+    """A thread that leaves because its own wait gave up sets the fault itself: another thread's
+    wait on the same barrier may just have succeeded, and the step would then go on with the
+    cells that were not written.  (Where the block decides together, one thread is enough.)"""
+    with open(os.path.join(CSRC, src)) as f:
+        text = re.sub(r"//[^\n]*", "", f.read())
+    for m in re.finditer(r"if \(!mbar_wait\([^;{]*\{", text):
+        assert re.match(r"\s*atomicExch\(&sc->fault, 1u\);", text[m.end():]), text[m.start():m.end() + 80]
