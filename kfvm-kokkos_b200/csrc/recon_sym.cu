@@ -444,7 +444,9 @@ __global__ void __launch_bounds__(Sym3<EQ>::THREADS, Sym3<EQ>::RESIDENT)
   double *quant = reinterpret_cast<double *>(smem + L::OFF_Q) + lane;
   double *red = reinterpret_cast<double *>(smem + L::OFF_R) + lane;      // GLM speeds [v][2][lane]
   unsigned *mask = reinterpret_cast<unsigned *>(smem + L::OFF_M);
-  const int i0 = (int)(blockIdx.x * L::BX), j = (int)blockIdx.y;
+  // the rows of cells are numbered along blockIdx.x: a grid may have more than 65535 of them in y
+  const unsigned nbx = (unsigned)(g.nx + L::BX - 1) / L::BX;
+  const int j = (int)(blockIdx.x / nbx), i0 = (int)((blockIdx.x - (unsigned)j * nbx) * L::BX);
   const int k0 = (int)blockIdx.z * zc, k1 = k0 + zc < (int)g.nz ? k0 + zc : (int)g.nz;
   using Ring = PlaneRing<L::RING>;
   const int last = k1 + 1;
@@ -876,7 +878,7 @@ static cudaError_t sym3(const ReconSymArgs &a, const CUtensorMap &umap, const Gr
       off.f[d][o] = (q * L::NV * g.nface[d] + str) * 8;
       off.w[d][o] = q * g.nface[d] + str;
     }
-  const dim3 grid((unsigned)bx, (unsigned)by, (unsigned)((g.nz + zc - 1) / zc));
+  const dim3 grid((unsigned)(bx * by), 1u, (unsigned)((g.nz + zc - 1) / zc));
   return launch_chain(g.chain, recon_sym3_kernel<EQ>, grid, dim3(L::THREADS), L::BYTES, s, umap, g, w, off, (int)zc, a.wantInd,
                       a.F[0], a.F[1], a.F[2], a.W[0], a.W[1], a.W[2], a.src, a.status, a.lamvel, a.bnd, a.sc);
 }

@@ -82,3 +82,19 @@ def test_block_edges_against_oracle(dim, nx, ny, nz, eq, gpu, product_lib, oracl
     assert np.array_equal(ag, ao)
     assert np.allclose(tg, to, rtol=0, atol=1e-10)
     assert np.abs(rg - ro).max() <= 1e-10 * np.abs(ro).max()
+
+
+@pytest.mark.gpu
+def test_more_rows_than_a_launch_has_in_y(gpu, product_lib, oracle_lib):
+    """65600 rows of cells in y, above the 65535 of a launch's second dimension.  The cells are
+    1 / 65600 high: fluxes of a few units with 20 roundings of 2^-53 each, and initial values
+    one rounding apart, differ by 1e-14, and the right-hand side by that times 65600."""
+    cfg = abi.make_config(3, abi.KFVM_EQ_HYDRO, 3, 65600, 3, bc=["periodic"] * 6, gamma=1.4)
+    g, o = product_lib.Solver(cfg), oracle_lib.OracleSolver(cfg)
+    for s in (g, o):
+        s.set_indicator(abi.KFVM_IND_NONE)
+        s.init_ic(abi.KFVM_IC_SMOOTH_WAVE)
+    rg, vg = g.eval_rhs()
+    ro, vo = o.eval_rhs()
+    assert abs(vg - vo) <= 1e-12 * abs(vo)
+    assert np.abs(rg - ro).max() <= 1e-9 * np.abs(ro).max()
