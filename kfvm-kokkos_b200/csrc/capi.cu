@@ -286,6 +286,7 @@ struct kfvm_solver {
   bool dmapOk = false;
   kfvm::SymW symw;
   bool symOk = false;
+  int symPlanes = 1;  // planes of a block in 3D
   int64_t nRhs = 0, nWenoLast = 0;
   int nTS = 1;
   double dmin = 0.0;
@@ -568,7 +569,7 @@ int eval_front(kfvm_solver *s, int b) {
                                     s->lamvel, s->bnd, s->sc, st);
            }
            if (s->symOk) {
-             const ReconSymArgs a{wantInd, s->F, s->W, s->src, s->status, s->lamvel, s->bnd, s->sc};
+             const ReconSymArgs a{wantInd, s->symPlanes, s->F, s->W, s->src, s->status, s->lamvel, s->bnd, s->sc};
              return launch_recon_sym(dim, eq, a, s->dmap[b], s->g, s->symw, st);
            }
            return launch_recon(dim, eq, s->Ub[b], s->dmapOk ? &s->dmap[b] : nullptr, s->g, s->dS, wantInd, s->F,
@@ -1053,6 +1054,7 @@ int kfvm_create(const kfvm_config *cfg, kfvm_solver **out) {
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
     if (nsm > 0) s->nsm = nsm;
+    if (s->symOk && s->dim == 3) s->symPlanes = recon_sym_planes(s->eq, g, s->nsm);
   }
   {
     const int64_t nb = std::max(std::max(stage_blocks(g), errest_blocks(g.n)), forcing_blocks(g));

@@ -103,6 +103,7 @@ cudaError_t launch_bounds(int dim, int eq, const double *U, const Grid &g, doubl
 // Two Gauss points per direction, not SR (recon_sym.cu): umap is recon_sym_state_map of U
 struct ReconSymArgs {
   int wantInd;
+  int planes;  // of a block in 3D (recon_sym_planes)
   double *const *F;
   float *const *W;
   double *src;
@@ -114,6 +115,8 @@ struct ReconSymArgs {
 cudaError_t launch_recon_sym(int dim, int eq, const ReconSymArgs &a, const CUtensorMap &umap, const Grid &g,
                              const SymW &w, cudaStream_t s);
 int recon_sym_state_map(CUtensorMap *map, const double *U, const Grid &g, int dim, int nv);
+// host: the planes that a block of the 3D form marches through, for nsm multiprocessors
+int recon_sym_planes(int eq, const Grid &g, int nsm);
 // host: the parity weights of a stencil with two Gauss points; nonzero where the
 // weights of mirrored points are not mirror images
 int fill_sym_weights(const kfvm_stencil &st, bool interior, SymW &out);

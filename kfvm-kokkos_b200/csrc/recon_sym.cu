@@ -849,17 +849,14 @@ int recon_sym_state_map(CUtensorMap *map, const double *U, const Grid &g, int di
   return encode_tensor_map_8b(map, U, 4, dims, strides, box);
 }
 
-template <int EQ>
-static cudaError_t sym3(const ReconSymArgs &a, const CUtensorMap &umap, const Grid &g, const SymW &w, cudaStream_t s) {
-  using L = Sym3<EQ>;
-  static const cudaError_t attr =
-      cudaFuncSetAttribute(recon_sym3_kernel<EQ>, cudaFuncAttributeMaxDynamicSharedMemorySize, L::BYTES);
-  if (attr != cudaSuccess) return attr;
-  const int64_t bx = (g.nx + L::BX - 1) / L::BX, by = g.ny;
-  // planes per block: a chunk costs about 2.5 planes' time besides its own planes (the
-  // first loads and footprints), and the blocks run in waves of the resident ones: the
-  // chunk count with the least waves times chunk cost
-  const int64_t cols = bx * by, slots = 148 * L::RESIDENT;
+// A chunk costs about 2.5 planes' time besides its own planes (the first loads and
+// footprints), and the blocks run in waves of the resident ones: the chunk count with the
+// least waves times chunk cost.  The choice depends little on that cost: with 0.5 and 1.5
+// planes nine sizes from 32^3 to 256 x 256 x 40 take the same times within 6 %, with 3.5
+// 160^3 takes 1.42 instead of 1.28 ms, with 8 the grid of 97 x 75 x 51 0.22 instead of 0.17.
+int recon_sym_planes(int eq, const Grid &g, int nsm) {
+  const int64_t cols = (g.nx + Sym3<EQ_HYDRO>::BX - 1) / Sym3<EQ_HYDRO>::BX * g.ny;
+  const int64_t slots = (int64_t)nsm * (eq == EQ_GLM ? Sym3<EQ_GLM>::RESIDENT : Sym3<EQ_HYDRO>::RESIDENT);
   int64_t zc = g.nz;
   double best = 1e300;
   for (int64_t n = 1; n <= g.nz; n++) {
@@ -870,6 +867,15 @@ static cudaError_t sym3(const ReconSymArgs &a, const CUtensorMap &umap, const Gr
       zc = len;
     }
   }
+  return (int)zc;
+}
+
+template <int EQ>
+static cudaError_t sym3(const ReconSymArgs &a, const CUtensorMap &umap, const Grid &g, const SymW &w, cudaStream_t s) {
+  using L = Sym3<EQ>;
+  static const cudaError_t attr =
+      cudaFuncSetAttribute(recon_sym3_kernel<EQ>, cudaFuncAttributeMaxDynamicSharedMemorySize, L::BYTES);
+  if (attr != cudaSuccess) return attr;
   SymOff off;
   for (int d = 0; d < 3; d++)
     for (int o = 0; o < 8; o++) {
@@ -878,8 +884,8 @@ static cudaError_t sym3(const ReconSymArgs &a, const CUtensorMap &umap, const Gr
       off.f[d][o] = (q * L::NV * g.nface[d] + str) * 8;
       off.w[d][o] = q * g.nface[d] + str;
     }
-  const dim3 grid((unsigned)(bx * by), 1u, (unsigned)((g.nz + zc - 1) / zc));
-  return launch_chain(g.chain, recon_sym3_kernel<EQ>, grid, dim3(L::THREADS), L::BYTES, s, umap, g, w, off, (int)zc, a.wantInd,
+  const dim3 grid((unsigned)((g.nx + L::BX - 1) / L::BX * g.ny), 1u, (unsigned)((g.nz + a.planes - 1) / a.planes));
+  return launch_chain(g.chain, recon_sym3_kernel<EQ>, grid, dim3(L::THREADS), L::BYTES, s, umap, g, w, off, a.planes, a.wantInd,
                       a.F[0], a.F[1], a.F[2], a.W[0], a.W[1], a.W[2], a.src, a.status, a.lamvel, a.bnd, a.sc);
 }
 
