@@ -2140,8 +2140,12 @@ __global__ void __launch_bounds__(128)
         const double uh = uha[v] + co.bhatDt * r[v], u = st[v];
         Uhat[v * g.n + c] = uh;
         hasNan = hasNan || isnan(u);
-        // (SR keeps the quotient: the last bit of the step size decides its theta in uniform gas)
-        const double tol = atol + rtol * fmax(fabs(u), fabs(uh)), e = EQ == EQ_SR ? (u - uh) / tol : (u - uh) * rcp_nr(tol);
+        // The refined reciprocal holds for normal values only, not for an infinite tolerance or
+        // none at all.  (SR keeps the quotient: the last bit of the step size decides its
+        // theta in uniform gas)
+        const double tol = atol + rtol * fmax(fabs(u), fabs(uh));
+        const bool normal = EQ != EQ_SR && tol > 1e-290 && tol < 1e290;
+        const double e = normal ? (u - uh) * rcp_nr(tol) : (u - uh) / tol;
         err += e * e;
       }
       pos = hasNan ? -1.0 : E::positivity(st);

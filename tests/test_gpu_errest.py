@@ -43,3 +43,21 @@ def test_err_est_matches_formula(name, scale, gpu, product_lib):
     _, pos2 = s.err_est(du2.data_ptr(), duh.data_ptr())
     assert pos2 == -1.0
     s.close()
+
+
+@pytest.mark.parametrize("name,scale", [("isentropic_vortex", 16), ("orszag_tang", 16)])
+@pytest.mark.parametrize("atol,rtol", [(1e-4, 1e-4), (np.inf, 1e-4), (1e300, 0.0), (1e290, 1e290), (0.0, 1e-4)])
+def test_step_error_at_extreme_tolerances(name, scale, atol, rtol, gpu, product_lib, oracle_lib):
+    """The error estimate of a step where the tolerance has no normal reciprocal: infinite, near
+    the ends of the range, zero (0 / 0 of a variable that is 0 everywhere: not a number, and the
+    step size grows by the fixed factor).  u - uhat of a first step is about 1e-9 of u, so
+    a rounding of u moves the estimate by 1e-7."""
+    cfg, ic = abi.workload(name, scale=scale, steps=1)
+    cfg.atol, cfg.rtol = atol, rtol
+    g, o = product_lib.Solver(cfg), oracle_lib.OracleSolver(cfg)
+    o.init_ic(ic)
+    g.set_state(o.get_state())
+    for _ in range(2):
+        ig, io = g.take_step(), o.take_step()
+        assert ig.accepted == io.accepted
+        np.testing.assert_allclose([ig.err_est, ig.dt], [io.err_est, io.dt], rtol=1e-4)
