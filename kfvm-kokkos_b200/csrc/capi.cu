@@ -976,7 +976,7 @@ int kfvm_create(const kfvm_config *cfg, kfvm_solver **out) {
   g.gamma = cfg->gamma;
   g.rs = cfg->rs;
   g.nq = cfg->nq;
-  g.chain = cfg->dim == 2 || g.n <= (1 << 16);
+  g.chain = cfg->dim == 2 || (g.n <= (1 << 16) && cfg->eq != KFVM_EQ_SRHYDRO);  // launch_chain has the times
   s->dmin = cfg->dim == 2 ? std::fmin(g.dx, g.dy) : std::fmin(g.dx, std::fmin(g.dy, g.dz));
 
   DevStencil hS;

@@ -1073,7 +1073,10 @@ struct HeavyShape {
 };
 
 // (2D, five variables: four blocks per SM at 96 registers instead of two at 148 took the
-// SR four-quadrant problem at 512^2 from 0.46 to 0.32 ms per evaluation)
+// SR four-quadrant problem at 512^2 from 0.46 to 0.32 ms per evaluation; with three Gauss
+// points, where it spills 16 to 40 bytes, the pass with WENO everywhere takes 0.234 ms for
+// Euler 512^2 and 0.102 for SR 256^2, against 0.393 and 0.149 of the form before it with
+// two blocks)
 template <int DIM, int EQ, int NQ>
 __global__ void __launch_bounds__(HeavyShape<DIM, EQ, NQ>::CELLS * Eos<EQ>::NV, Eos<EQ>::NV > 5 ? 1 : (DIM == 2 ? 4 : 2))
     heavy_var_kernel(const double *U, Grid g, const DevStencil *__restrict__ S,

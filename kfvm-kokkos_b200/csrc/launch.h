@@ -40,11 +40,15 @@ struct StageArgs {
 // array that nothing else is said to name.  So in these kernels only tables written at
 // creation (DevStencil) and arrays that the kernel itself only writes are __restrict__.
 //
-// early: Grid::chain, which is set in 2D and up to 2^16 cells in 3D.  Whole passes with
-// and without: Euler 2D 32^2 0.58 and 0.83 ms, 1024^2 12.9 and 13.3, 2048^2 26.0 and 26.3;
-// Euler 3D 40^3 4.50 and 4.65, but 50^3 5.18 and 4.99, 256^3 245 and 232: the 3D kernels
-// fill the SMs' shared memory and registers, and the next kernel's waiting blocks do not
-// sit beside them for free.
+// early: Grid::chain, which is set in 2D and, except for SR, up to 2^16 cells in 3D.  Steps in
+// us, early and not, at 32^2, 256^2 and 1024^2: Euler 149 and 194, 207 and 246, 1250 and 1300;
+// Navier-Stokes 163 and 207, 215 and 248, 1350 and 1415; GLM-MHD 185 and 220, 268 and 330, 2650
+// and 2725; SR 393 and 438, 740 and 748, 7655 and 7710.  In 3D at 16^3, 32^3 and 40^3: Euler
+// 284 and 292, 396 and 406, 585 and 604; Navier-Stokes 150 and 202, 222 and 274, 400 and 424;
+// GLM-MHD 319 and 370, 707 and 732, 1134 and 1149; but SR 1265 and 1200 at 2000 x 4 x 4, 2210 and
+// 2144 at 1000 x 8 x 8, and larger grids (whole passes of Euler 50^3 5.18 and 4.99 ms, 256^3 245
+// and 232): the 3D kernels fill the SMs' shared memory and registers, SR's recovery most of
+// all, and the next kernel's waiting blocks do not sit beside them for free.
 template <class... Params, class... Args>
 cudaError_t launch_chain(bool early, void (*kernel)(Params...), dim3 grid, dim3 block, size_t smem, cudaStream_t s,
                          const Args &...args) {
