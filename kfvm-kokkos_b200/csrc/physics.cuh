@@ -153,9 +153,6 @@ struct Eos {
   __device__ __forceinline__ static double pres(double g, const double *U) {
     return (g - 1.0) * eint(U);
   }
-  __device__ __forceinline__ static double soundspeed(double g, const double *U) {
-    return sqrt(g * pres(g, U) / U[DENS]);
-  }
   // KXRCF indicator variable p / rho^gamma (SR: the density D, SRHydro_EOS.H:225-228)
   __device__ __forceinline__ static double weno(double g, const double *U) {
     if constexpr (EQ == EQ_SR) return U[DENS];
@@ -236,23 +233,6 @@ struct Eos {
     }
     return fmin(U[DENS], eint(U));
   }
-  __device__ __forceinline__ static void cons2prim(double g, const double *U, double *V) {
-    if constexpr (EQ == EQ_SR) {
-      sr::cons2prim(g, U, V);
-      return;
-    }
-    V[0] = U[DENS];
-    V[1] = U[MOMX] / U[DENS];
-    V[2] = U[MOMY] / U[DENS];
-    V[3] = U[MOMZ] / U[DENS];
-    V[4] = pres(g, U);
-    if constexpr (EQ == EQ_GLM) {
-      V[5] = U[MAGX];
-      V[6] = U[MAGY];
-      V[7] = U[MAGZ];
-      V[8] = U[PSI];
-    }
-  }
   __device__ __forceinline__ static double fastMagSonic(double g, const double *U, double bl) {
     const double asq = g * pres(g, U) / U[DENS];
     const double bsq = 2.0 * prsb(U) / U[DENS];
@@ -299,10 +279,6 @@ struct Eos {
       F[bo[2]] = vx * bz - vz * bx;
       F[PSI] = ch * bx;
     }
-  }
-
-  __device__ __forceinline__ static double roeAvg(double rL, double rR, double qL, double qR) {
-    return (qL * sqrt(rL) + qR * sqrt(rR)) / (sqrt(rL) + sqrt(rR));
   }
 
   // GLM-MHD primitives and fast speed with the density reciprocal ir taken once

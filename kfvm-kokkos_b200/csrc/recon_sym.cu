@@ -37,7 +37,6 @@
 #include <algorithm>
 #include <cmath>
 #include <cstring>
-#include <type_traits>
 
 #include "kernels.cuh"
 #include "launch.h"
@@ -47,14 +46,8 @@
 
 namespace kfvm {
 
-template <int DIM>
-struct SymShape {
-  static constexpr int NS = DIM == 3 ? 33 : 13;  // stencil combinations
-  static constexpr int NP = 1 << DIM;            // points of a group (one face direction, or the interior)
-};
-
-// Stencil combinations, in the order of the weights (fill_sym_weights): ld(dx, dy, dz)
-// is the difference to the cell's value at that offset, and the value itself at (0, 0, 0).  The combinations come grouped by parity: even in
+// Stencil combinations, in the order of the weights (fill_sym_weights), of differences to the
+// cell's value (the value itself comes first).  They come grouped by parity: even in
 // all axes, odd in x, odd in y, (odd in z, in x and y, in x and z, in y and z, in all).
 // In 3D the combinations within a plane (x and y) are formed once per plane, as
 // differences to the cell's own value in that plane, and serve the three planes of cells
@@ -111,22 +104,23 @@ __device__ __forceinline__ void sym_combine(const double *u, const SymPlane &m, 
   s[24] = fma(2.0, s[21], s[24]);
   s[25] = fma(4.0, s[21], s[25]);
 }
+// in 2D: ld(dx, dy) is the difference at that offset, and the value itself at (0, 0)
 template <class Ld>
 __device__ __forceinline__ void sym_combine(Ld ld, double (&s)[13]) {
-  s[0] = ld(0, 0, 0);
-  double a = ld(1, 0, 0), b = ld(-1, 0, 0);
+  s[0] = ld(0, 0);
+  double a = ld(1, 0), b = ld(-1, 0);
   s[1] = a + b;
   s[6] = a - b;
-  a = ld(0, 1, 0), b = ld(0, -1, 0);
+  a = ld(0, 1), b = ld(0, -1);
   s[2] = a + b;
   s[9] = a - b;
-  a = ld(2, 0, 0), b = ld(-2, 0, 0);
+  a = ld(2, 0), b = ld(-2, 0);
   s[3] = a + b;
   s[7] = a - b;
-  a = ld(0, 2, 0), b = ld(0, -2, 0);
+  a = ld(0, 2), b = ld(0, -2);
   s[4] = a + b;
   s[10] = a - b;
-  const double pp = ld(1, 1, 0), pm = ld(1, -1, 0), mp = ld(-1, 1, 0), mm = ld(-1, -1, 0);
+  const double pp = ld(1, 1), pm = ld(1, -1), mp = ld(-1, 1), mm = ld(-1, -1);
   const double e = pp + pm, f = pp - pm, g = mp + mm, h = mp - mm;
   s[5] = e + g;
   s[8] = e - g;
@@ -134,7 +128,7 @@ __device__ __forceinline__ void sym_combine(Ld ld, double (&s)[13]) {
   s[12] = f - h;
 }
 
-// The NP points of a group from its weights (w[0] is not used): f[o], bit d of o set where the point
+// The 8 (4) points of a group from its weights (w[0] is not used): f[o], bit d of o set where the point
 // lies on the positive side of axis d.
 __device__ __forceinline__ void sym_points(const double *w, const double (&s)[33], double (&f)[8]) {
   auto dot = [&](int b, int n) {
@@ -186,33 +180,35 @@ __device__ __forceinline__ constexpr int sym_inner_q(int o) {
   return DIM == 2 ? 2 * x + y : (2 * x + y) * 2 + z;
 }
 
-// What a cell's thread needs besides its stencil values.
-template <int DIM>
-struct SymCell {
+// The limiter's bounds of a cell.
+struct SymBounds {
   double minDens, maxDens, minEint;
+};
+// What a cell's thread needs besides its stencil values in 2D.
+struct SymCell {
+  SymBounds bd;
   int64_t c;        // cell index
-  int64_t fidx[3];  // its low face per axis
-  int64_t fstr[3];  // from there to the high face
+  int64_t fidx[2];  // its low face per axis
+  int64_t fstr[2];  // from there to the high face
 };
 
-// One cell: ld(v, dx, dy, dz) gives variable v at an offset.  Writes the face states
+// One cell in 2D: ld(v, dx, dy) gives variable v at an offset.  Writes the face states
 // (and the interior points), the indicator and the cell's status.
 //
 // A cell whose states do not lie inside the limiter's bounds with a margin of
 // rounding goes to the heavy pass, which decides exactly (theta stays 1 there when
 // the states are inside after all), so the kinetic energy needs no IEEE division here.
-template <int DIM, int EQ, class Ld>
-__device__ __forceinline__ void sym_cell(Ld ld, const SymW &w, const Grid &g, const SymCell<DIM> &cl, int wantInd,
-                                         double *const (&F)[3], float *const (&W)[3], double *__restrict__ src,
+template <int EQ, class Ld>
+__device__ __forceinline__ void sym_cell(Ld ld, const SymW &w, const Grid &g, const SymCell &cl, int wantInd,
+                                         double *const (&F)[2], float *const (&W)[2], double *__restrict__ src,
                                          uint8_t *__restrict__ status, double2 *__restrict__ lamvel) {
   using E = Eos<EQ>;
-  using Sh = SymShape<DIM>;
-  constexpr int NV = E::NV, NQF = DIM == 2 ? 2 : 4, NP = Sh::NP, NS = Sh::NS;
+  constexpr int DIM = 2, NV = E::NV, NQF = 2, NP = 4, NS = 13;
   bool inside = true;
   double lam = 0.0, vel = 0.0;
   auto combine = [&](int v, double (&s)[NS]) {
-    const double c = ld(v, 0, 0, 0);
-    sym_combine([&](int dx, int dy, int dz) { return dx == 0 && dy == 0 && dz == 0 ? c : ld(v, dx, dy, dz) - c; }, s);
+    const double c = ld(v, 0, 0);
+    sym_combine([&](int dx, int dy) { return dx == 0 && dy == 0 ? c : ld(v, dx, dy) - c; }, s);
   };
   // the points of face direction d for variable v, stored; f[o] as sym_points
   auto points = [&](int d, int v, const double (&s)[NS], double (&f)[NP]) {
@@ -238,7 +234,7 @@ __device__ __forceinline__ void sym_cell(Ld ld, const SymW &w, const Grid &g, co
   if constexpr (EQ != EQ_GLM) {
     // momenta (their squares), density (kinetic energy, power of the indicator), energy
     double acc[DIM * NP];
-    std::conditional_t<DIM == 2, double, float> pw[DIM * NP];
+    double pw[DIM * NP];
 #pragma unroll
     for (int t = 0; t < DIM * NP; t++) acc[t] = 0.0;
 #pragma unroll 1
@@ -261,7 +257,7 @@ __device__ __forceinline__ void sym_cell(Ld ld, const SymW &w, const Grid &g, co
 #pragma unroll
         for (int o = 0; o < NP; o++) {
           double &a = acc[d * NP + o];
-          inside = inside && f[o] > cl.minDens && f[o] < cl.maxDens && f[o] > 0.0;
+          inside = inside && f[o] > cl.bd.minDens && f[o] < cl.bd.maxDens && f[o] > 0.0;
           a = 0.5 * a * rcp_nr(f[o]);
           if (wantInd) pw[d * NP + o] = E::template weno_power<DIM>(g.gamma, f[o]);
         }
@@ -276,7 +272,7 @@ __device__ __forceinline__ void sym_cell(Ld ld, const SymW &w, const Grid &g, co
 #pragma unroll
         for (int o = 0; o < NP; o++) {
           const double a = acc[d * NP + o], ei = f[o] - a;
-          inside = inside && ei - cl.minEint > 8.9e-16 * (fabs(a) + fabs(ei)) + 1e-300;
+          inside = inside && ei - cl.bd.minEint > 8.9e-16 * (fabs(a) + fabs(ei)) + 1e-300;
           if (wantInd) store_ind(d, o, E::template weno_from_power<DIM>((g.gamma - 1.0) * ei, pw[d * NP + o]));
         }
       }
@@ -288,7 +284,7 @@ __device__ __forceinline__ void sym_cell(Ld ld, const SymW &w, const Grid &g, co
     for (int d = 0; d <= DIM; d++) {
       // sums over the variables as they come: momenta, magnetic field, psi, density, energy
       double m2[NP], b2[NP], mx[NP], bx[NP], ps[NP], ir[NP];
-      std::conditional_t<DIM == 2, double, float> pw[NP];
+      double pw[NP];
 #pragma unroll
       for (int o = 0; o < NP; o++) m2[o] = b2[o] = mx[o] = bx[o] = ps[o] = ir[o] = 0.0, pw[o] = 0;
 #pragma unroll 1
@@ -314,12 +310,12 @@ __device__ __forceinline__ void sym_cell(Ld ld, const SymW &w, const Grid &g, co
           } else if (v == PSI) {
             ps[o] = 0.5 * f[o] * f[o];
           } else if (v == DENS) {
-            inside = inside && f[o] > cl.minDens && f[o] < cl.maxDens && f[o] > 0.0;
+            inside = inside && f[o] > cl.bd.minDens && f[o] < cl.bd.maxDens && f[o] > 0.0;
             ir[o] = rcp_nr(f[o]);
             if (wantInd && d < DIM) pw[o] = E::template weno_power<DIM>(g.gamma, f[o]);
           } else {
             const double other = 0.5 * b2[o] + 0.5 * m2[o] * ir[o] + ps[o], ei = f[o] - other;
-            inside = inside && ei - cl.minEint > 8.9e-16 * (fabs(other) + fabs(ei)) + 1e-300;
+            inside = inside && ei - cl.bd.minEint > 8.9e-16 * (fabs(other) + fabs(ei)) + 1e-300;
             if (d < DIM) {
               const double p = (g.gamma - 1.0) * ei;
               if (wantInd) store_ind(d, o, E::template weno_from_power<DIM>(p, pw[o]));
@@ -360,31 +356,13 @@ struct SymExt {
 };
 // PositivityPreserve_K bounds (Common_K.H:331-380) from the neighbourhood's extrema
 // and twice the velocity divergence
-template <int DIM>
-__device__ __forceinline__ void sym_bounds(const SymExt &x, double div2, SymCell<DIM> &cl) {
+__device__ __forceinline__ SymBounds sym_bounds(const SymExt &x, double div2) {
   const double snd = sqrt_nr(x.c2Min), divV = div2 / 2.0;
   double kappa = 0.2;
   // (the IEEE quotient: cold gas has snd = 0, and +-infinity decides)
   const double eta = fmin(1.0, fmax(0.0, -(kappa * snd + divV) / (kappa * snd)));
   kappa *= (1.0 - eta);
-  cl.maxDens = x.rMax * (1.0 + kappa);
-  cl.minDens = x.rMin * (1.0 - kappa);
-  cl.minEint = x.eMin * (1.0 - kappa);
-}
-
-// the cell's index, faces and stored bounds
-template <int DIM>
-__device__ __forceinline__ void sym_locate(const Grid &g, int64_t i, int64_t j, int64_t k, double *__restrict__ bnd,
-                                           SymCell<DIM> &cl) {
-  cl.c = (k * g.ny + j) * g.nx + i;
-#pragma unroll
-  for (int d = 0; d < DIM; d++) {
-    cl.fidx[d] = (k * g.fdim[d][1] + j) * g.fdim[d][0] + i;
-    cl.fstr[d] = d == 0 ? 1 : (d == 1 ? g.fdim[1][0] : g.fdim[2][0] * g.fdim[2][1]);
-  }
-  bnd[cl.c] = cl.minDens;  // for the heavy pass
-  bnd[g.n + cl.c] = cl.maxDens;
-  bnd[2 * g.n + cl.c] = cl.minEint;
+  return {x.rMin * (1.0 - kappa), x.rMax * (1.0 + kappa), x.eMin * (1.0 - kappa)};
 }
 
 // Where the points of a cell go, as byte offsets from the cell's low face at variable v
@@ -432,7 +410,7 @@ __global__ void __launch_bounds__(Sym3<EQ>::THREADS, Sym3<EQ>::RESIDENT)
   pdl_begin();
   using L = Sym3<EQ>;
   using E = Eos<EQ>;
-  constexpr int NV = L::NV, TX = L::TX, TN = L::TN, PX = L::PX, PN = L::PN, NQF = 4;
+  constexpr int NV = L::NV, TX = L::TX, TN = L::TN, PX = L::PX, PN = L::PN;
   constexpr double big = 1.7976931348623157e308;
   extern __shared__ __align__(128) uint8_t smem[];
   double *ring = reinterpret_cast<double *>(smem);
@@ -599,15 +577,14 @@ __global__ void __launch_bounds__(Sym3<EQ>::THREADS, Sym3<EQ>::RESIDENT)
     double ap = 0.0, bp = 0.0;
     if (k + 1 < k1) survey(ring + sq, 1 - par, ap, bp);
     if (v == ETOT) {
-      SymCell<3> cl;
-      sym_bounds<3>(SymExt{quant[0], quant[32], quant[64], quant[96]}, quant[128], cl);
-      quant[5 * 32] = cl.minDens > 0.0 ? cl.minDens : 0.0;
-      quant[6 * 32] = cl.maxDens;
-      quant[7 * 32] = cl.minEint;
+      const SymBounds bd = sym_bounds(SymExt{quant[0], quant[32], quant[64], quant[96]}, quant[128]);
+      quant[5 * 32] = bd.minDens > 0.0 ? bd.minDens : 0.0;
+      quant[6 * 32] = bd.maxDens;
+      quant[7 * 32] = bd.minEint;
       if (live) {
-        bnd[wb[2]] = cl.minDens;  // for the heavy pass
-        bnd[g.n + wb[2]] = cl.maxDens;
-        bnd[2 * g.n + wb[2]] = cl.minEint;
+        bnd[wb[2]] = bd.minDens;  // for the heavy pass
+        bnd[g.n + wb[2]] = bd.maxDens;
+        bnd[2 * g.n + wb[2]] = bd.minEint;
       }
     }
     // ---- the contraction of this warp's variable
@@ -764,13 +741,21 @@ __global__ void __launch_bounds__(Sym2<EQ>::THREADS, Sym2<EQ>::RESIDENT)
     }
   const double *ir = foot + 2 * PN + pown, *mx = u + MOMX * TN, *my = u + MOMY * TN;
   const double div2 = (mx[1] * ir[1] - mx[-1] * ir[-1]) + (my[TX] * ir[PX] - my[-TX] * ir[-PX]);
-  SymCell<2> cl;
-  sym_bounds<2>(x, div2, cl);
-  sym_locate<2>(g, i, j, 0, bnd, cl);
-  double *const F[3] = {F0, F1, nullptr};
-  float *const W[3] = {W0, W1, nullptr};
-  sym_cell<2, EQ>([&](int v, int dx, int dy, int) { return u[v * TN + dy * TX + dx]; }, w, g, cl, wantInd, F, W, src,
-                  status, lamvel);
+  SymCell cl;
+  cl.bd = sym_bounds(x, div2);
+  cl.c = j * g.nx + i;
+#pragma unroll
+  for (int d = 0; d < 2; d++) {
+    cl.fidx[d] = j * g.fdim[d][0] + i;
+    cl.fstr[d] = d == 0 ? 1 : g.fdim[1][0];
+  }
+  bnd[cl.c] = cl.bd.minDens;  // for the heavy pass
+  bnd[g.n + cl.c] = cl.bd.maxDens;
+  bnd[2 * g.n + cl.c] = cl.bd.minEint;
+  double *const F[2] = {F0, F1};
+  float *const W[2] = {W0, W1};
+  sym_cell<EQ>([&](int v, int dx, int dy) { return u[v * TN + dy * TX + dx]; }, w, g, cl, wantInd, F, W, src, status,
+               lamvel);
 }
 
 // ---------------------------------------------------------------------------
