@@ -1765,7 +1765,7 @@ __global__ void __launch_bounds__(RiemannShape<DIM, EQ, NQ>::THREADS, RiemannSha
 // Bound by its loads (136 face and interior values in 3D): the places of a cell's faces
 // and their boundary redirection are worked out once per direction, and the terms are
 // summed over the points before they meet div B, which is the same for all of them
-// (per value before: stage kernel 0.29 ms at 1024^2 and 0.47 ms at 96^3; now 0.175 and 0.26 ms).
+// (per value before: stage kernel 0.29 ms a launch at 1024^2 and 0.47 ms at 96^3; now 0.12 and 0.22 ms).
 template <int DIM, int NQ>
 __device__ __forceinline__ void glm_sources(const double *Uc, const Grid &g, int64_t i, int64_t j,
                                             int64_t k, int64_t c, const double *F0,
@@ -2106,8 +2106,8 @@ __global__ void __launch_bounds__(128)
       for (int v = 0; v < NV; v++) K[v * g.n + c] = r[v];
     } else if (mode == STAGE_UPDATE) {
       // every load before the stores, which may alias them (the registers this takes, 72 instead
-      // of 40 for Euler, cost nothing: per launch Sod 256^3 0.64 -> 0.56 ms, Navier-Stokes
-      // 160^3 0.30 -> 0.24)
+      // of 40 for Euler, cost nothing: per evaluation Sod 256^3 0.79 -> 0.70 ms, Navier-Stokes
+      // 160^3 0.37 -> 0.30)
       double u[NV], uh[NV], ut[NV], up[NV];
 #pragma unroll
       for (int v = 0; v < NV; v++) {

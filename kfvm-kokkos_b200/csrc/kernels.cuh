@@ -12,15 +12,16 @@
 //                in-bounds linear cells, the compacted list of heavy cells
 //   heavy        WENO-AO and/or the full positivity limiter on the listed cells
 //                (KernelWenoRecon_K, PositivityPreserve_K)
-//   riemann<d>   one thread per face point: HLLC/HLL/LLF, quadrature weighted flux
-//                sum per face, max wave speed                 (RiemannSolver*_K)
+//   riemann      one thread per face point of every direction: HLLC/HLL/LLF, quadrature
+//                weighted flux sum per face, max wave speed   (RiemannSolver*_K)
 //   stage        flux divergence (+ viscous terms, + GLM sources), fused with the
 //                low-storage FSAL register update and the error estimate
 //                (IntegrateRHS_K, Viscosity_K, SourceTerms_K, RKFSAL_*_K)
 // Reference: slug-cfd/kfvm-kokkos src/Solver.cpp:188-530 and the functors named above.
 //
 // Layouts in HBM (all FP64):
-//   U      [v][nz+2r][ny+2r][nx+2r]   padded SoA, r = 2 (2D: one z plane, no z halo)
+//   U      [v][nz+2r][ny+2r][px]      padded SoA, r = 2 (2D: one z plane, no z halo); px is
+//                                     nx+2r, rounded up to an even number
 //   faces  [slot][q][v][face]         per direction, face = (k*fy + j)*fx + i
 //   flux   [v][face]                  quadrature-weighted flux per face
 //   K, Uhat, Utmp [v][cell]           interior SoA, cell = (k*ny + j)*nx + i

@@ -32,12 +32,13 @@ enum { RS_LLF = 0, RS_HLL = 1, RS_HLLC = 2 };
 // (<= 5.5e-6), i.e. <= 1.8e-5 x ln 2 = 1.2e-5 relative after ex2; ex2.approx
 // (2^-22) and the FP32 roundings of p and rho add < 4e-7.
 constexpr double kWenoApproxEps = 2e-5;
-// Two face states whose components differ by at most kSameTol x their largest
-// component are treated as one state by the Riemann kernel (Eos::same_state): every
-// solver here is consistent, F(u, u) = F(u), and differs from F(u) by about
-// (wave speed) x |uR - uL| for nearby states, so the flux changes by less than
-// 1e-14 of its scale.  The reconstruction of a uniform region leaves such
-// rounding-level differences between the two sides of a face.
+// Three Gauss points, and SR: two face states whose components differ by at most
+// kSameTol x their largest component are treated as one state by the Riemann kernel
+// (Eos::same_state): every solver here is consistent, F(u, u) = F(u), and differs from
+// F(u) by about (wave speed) x |uR - uL| for nearby states, so the flux changes by less
+// than 1e-14 of its scale.  The direct sum leaves such rounding-level differences between
+// the two sides of a face in a uniform region; the parity form gives equal states there,
+// and only those are treated as one.
 constexpr double kSameTol = 1e-14;
 // bound on the relative error of the indicator stored in 2D: one rounding to FP32
 // (2^-24 = 5.97e-8) and the 1e-9 of Eos::weno_power64 (SR stores the rounded density)
@@ -346,7 +347,7 @@ struct Eos {
     return same;
   }
 
-  // Face with equal states (kSameTol): the physical flux, and the speed bound
+  // Face with equal states (same_state): the physical flux, and the speed bound
   // max(|sL|, |sR|) that the estimates give for equal states.  Euler / Navier-Stokes:
   // |u_n| + a (Hydro_Riemann.H:41-81 with uTil = u, aTil = a); SRHydro: the larger
   // magnitude of the state's two characteristic bounds (SRHydro_Riemann.H:39-77),

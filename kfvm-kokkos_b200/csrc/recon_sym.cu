@@ -24,8 +24,8 @@
 //
 // Bound by the issue rate (the point test and the indicator cost more instructions than
 // the contraction) and by the block's two barriers per plane.  Per launch, the direct sum
-// on the FP64 tensor instruction before: Euler 256^3 7.5 -> 5.3 ms, Navier-Stokes 160^3
-// 1.89 -> 1.31 ms, GLM-MHD 96^3 1.45 -> 0.72 ms, Euler 1024^2 0.186 -> 0.111 ms, GLM-MHD
+// on the FP64 tensor instruction before: Euler 256^3 7.5 -> 5.0 ms, Navier-Stokes 160^3
+// 1.89 -> 1.30 ms, GLM-MHD 96^3 1.45 -> 0.72 ms, Euler 1024^2 0.186 -> 0.111 ms, GLM-MHD
 // 1024^2 0.48 -> 0.30 ms.
 //
 // Special-relativistic hydrodynamics keeps the direct sum (recon_tma_kernel): its limiter
