@@ -1072,6 +1072,35 @@ struct HeavyShape {
                                   (size_t)T::NB * SUB * sizeof(int);
 };
 
+// smoothness indicators -> normalised nonlinear weights (createOmegas, Stencil_K.H:556-580)
+template <int EQ, int NSUB>
+__device__ __forceinline__ void weno_normalise(double (&om)[NSUB], const double (&gam)[NSUB]) {
+  double top = 0.0, tot = 0.0;
+#pragma unroll
+  for (int s = 0; s < NSUB; s++) top = om[s] > top ? om[s] : top;
+  if (EQ != EQ_SR && top <= 1e140) {
+#pragma unroll
+    for (int s = 0; s < NSUB; s++) {
+      om[s] = gam[s] * rcp_nr(om[s] * om[s] + 1.e-40);
+      tot += om[s];
+    }
+    const double itot = rcp_nr(tot);
+#pragma unroll
+    for (int s = 0; s < NSUB; s++) om[s] *= itot;
+  } else {
+    // The quotients for SR, where the rounding of a uniform blend decides theta, and where
+    // a divisor has no normal reciprocal: values above 1e70 (overflowing squares give weights
+    // of zero, or none that are numbers, and the limiter then takes the cell's average).
+#pragma unroll
+    for (int s = 0; s < NSUB; s++) {
+      om[s] = gam[s] / (om[s] * om[s] + 1.e-40);
+      tot += om[s];
+    }
+#pragma unroll
+    for (int s = 0; s < NSUB; s++) om[s] /= tot;
+  }
+}
+
 // (2D, five variables: four blocks per SM at 96 registers instead of two at 148 took the
 // SR four-quadrant problem at 512^2 from 0.46 to 0.32 ms per evaluation; with three Gauss
 // points, where it spills 16 to 40 bytes, the pass with WENO everywhere takes 0.234 ms for
@@ -1256,16 +1285,7 @@ __global__ void __launch_bounds__(HeavyShape<DIM, EQ, NQ>::CELLS * Eos<EQ>::NV, 
           gam[1] = (1.0 - gHi) * gLo;
 #pragma unroll
           for (int s = 2; s < T::NSUB; s++) gam[s] = (1.0 - gHi) * (1.0 - gLo) / (DIM == 2 ? 4.0 : 6.0);
-          double tot = 0.0;
-#pragma unroll
-          for (int s = 0; s < T::NSUB; s++) {
-            const double b2 = om[s] * om[s];  // (a finite divisor; NaN stays)
-            om[s] = gam[s] * rcp_nr((b2 > 1e280 ? 1e280 : b2) + 1.e-40);
-            tot += om[s];
-          }
-          const double itot = rcp_nr(tot);
-#pragma unroll
-          for (int s = 0; s < T::NSUB; s++) om[s] *= itot;
+          weno_normalise<EQ>(om, gam);
           double dep = 0.0;
           if (sig)
 #pragma unroll
@@ -1390,21 +1410,7 @@ __global__ void __launch_bounds__(HeavyShape<DIM, EQ, NQ>::CELLS * Eos<EQ>::NV, 
       gam[1] = (1.0 - gHi) * gLo;
 #pragma unroll
       for (int s = 2; s < T::NSUB; s++) gam[s] = (1.0 - gHi) * (1.0 - gLo) / (DIM == 2 ? 4.0 : 6.0);
-      double tot = 0.0;
-#pragma unroll
-      for (int s = 0; s < T::NSUB; s++) {
-        // (SR keeps the reference's quotients: the rounding of a uniform blend decides its theta)
-        const double b2 = om[s] * om[s];  // (otherwise: a finite divisor; NaN stays)
-        if constexpr (EQ == EQ_SR) om[s] = gam[s] / (b2 + 1.e-40);
-        else om[s] = gam[s] * rcp_nr((b2 > 1e280 ? 1e280 : b2) + 1.e-40);
-        tot += om[s];
-      }
-      const double itot = EQ == EQ_SR ? 1.0 : rcp_nr(tot);
-#pragma unroll
-      for (int s = 0; s < T::NSUB; s++) {
-        if constexpr (EQ == EQ_SR) om[s] /= tot;
-        else om[s] *= itot;
-      }
+      weno_normalise<EQ>(om, gam);
       double dep = 0.0;
       if (sig)
 #pragma unroll

@@ -355,3 +355,38 @@ def test_glm_equal_state_variant(dim, n, gpu, product_lib, oracle_lib):
     err = rel_l1(g.get_state(), o.get_state())
     assert np.all(err <= STEP_TOL), err
     g.close()
+
+
+@pytest.mark.parametrize("dim,eq", [(2, abi.KFVM_EQ_HYDRO), (3, abi.KFVM_EQ_HYDRO), (2, abi.KFVM_EQ_MHD_GLM),
+                                    (3, abi.KFVM_EQ_MHD_GLM)])
+@pytest.mark.parametrize("expo", [-140, -70, 60, 72, 76])
+def test_units_of_any_size(dim, eq, expo, gpu, product_lib, oracle_lib):
+    """The same gas in units in which density and energy are 1e-140 to 1e76: WENO's squared
+    smoothness indicators reach 1e308 at the top, and the weights' divisors leave the range of a
+    normal reciprocal from 1e70 on.  Velocities stay of order 1, so that the right-hand side scales
+    with the state."""
+    n = (20, 12, 9)[:dim]
+    cfg = abi.make_config(dim, eq, *n, rs=abi.KFVM_RS_HLLC if eq == abi.KFVM_EQ_HYDRO else abi.KFVM_RS_HLL,
+                          bc=["periodic"] * 6, gamma=1.5, weno_thresh=-1.0)
+    g, o = product_lib.Solver(cfg), oracle_lib.OracleSolver(cfg)
+    rng = np.random.default_rng(5)
+    k = np.arange(abi.ncells(cfg))
+    rho = np.where(k % 20 > 9, 1.0, 0.3) * (1 + 0.1 * rng.uniform(-1, 1, k.size))
+    p = np.where(k // 20 % 12 > 5, 1.0, 0.2) * (1 + 0.1 * rng.uniform(-1, 1, k.size))
+    v = 0.3 * rng.uniform(-1, 1, (3, k.size))
+    u = np.zeros((g.nv, k.size))
+    u[0], u[1:4], u[4] = rho, rho * v, p / 0.5 + 0.5 * rho * (v ** 2).sum(0)
+    u *= 10.0 ** expo
+    if eq == abi.KFVM_EQ_MHD_GLM:
+        b = 0.2 * rng.uniform(-1, 1, (3, k.size))
+        u[5:8] = b * 10.0 ** (expo / 2)
+        u[4] += 0.5 * (b ** 2).sum(0) * 10.0 ** expo
+    g.set_state(u)
+    o.set_state(u)
+    rg, vg = g.eval_rhs()
+    ro, vo = o.eval_rhs()
+    assert abs(vg - vo) <= 1e-12 * vo
+    scale = np.abs(ro).max(axis=1, keepdims=True)
+    assert np.all(np.abs(rg - ro) <= 1e-11 * np.where(scale > 0, scale, 1.0))
+    (_, tg), (_, to) = g.flags(), o.flags()
+    assert np.allclose(tg, to, rtol=0, atol=1e-10)
