@@ -409,6 +409,7 @@ __global__ void __launch_bounds__(DmmaTile<DIM>::THREADS, (DIM == 2 && NQ == 2 &
     mbar_init(bar, 1);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     mbar_arrive_expect_tx(bar, (uint32_t)(NV * D::N * 8));
+    global_acquire_for_copies();
 #pragma unroll
     for (int v = 0; v < NV; v++) tma_load_4d(smem_u32(smem + v * D::N * 8), &umap, i0, j0, k0, v, bar);
   }

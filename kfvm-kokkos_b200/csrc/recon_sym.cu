@@ -437,6 +437,7 @@ __global__ void __launch_bounds__(Sym3<EQ>::THREADS, Sym3<EQ>::RESIDENT)
   if (tid == 0) {
     for (int s = 0; s < L::RING; s++) mbar_init(bar + 8 * s, 1);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    global_acquire_for_copies();
     for (int p = k0 - 2; p <= Ring::started(k0, last); p++) issue(p);
   }
   __syncthreads();
@@ -709,6 +710,7 @@ __global__ void __launch_bounds__(Sym2<EQ>::THREADS, Sym2<EQ>::RESIDENT)
     mbar_init(bar, 1);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     mbar_arrive_expect_tx(bar, (uint32_t)sizeof(tile));
+    global_acquire_for_copies();
     tma_load_4d(smem_u32(tile), &umap, i0, j0, 0, 0, bar);
   }
   __syncthreads();

@@ -31,6 +31,13 @@ __device__ __forceinline__ void tma_prefetch_map(const CUtensorMap *map) {
   asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(map)) : "memory");
 }
 
+// Orders what earlier kernels stored in global memory, as pdl_begin's wait made it visible,
+// before the copies that this thread issues next (the end of a kernel does that by itself; a
+// kernel launched early begins before it).
+__device__ __forceinline__ void global_acquire_for_copies() {
+  asm volatile("fence.proxy.async.global;" ::: "memory");
+}
+
 // Orders this thread's ordinary accesses to shared memory before copies into it that are
 // issued behind the next barrier.  A barrier alone does not: a load whose value is not
 // needed yet may still wait in the load/store queue when the copy lands.

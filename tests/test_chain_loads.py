@@ -91,3 +91,17 @@ def test_reads_are_ordinary_loads_behind_the_wait(name):
             continue
         assert "const" not in p, p
         assert n in WRITTEN_ONLY[name], p
+
+
+def test_copies_are_ordered_behind_the_wait():
+    """What pdl_begin's wait makes visible, it makes visible to ordinary loads: the thread that
+    issues TMA copies of the predecessors' arrays passes a proxy fence first."""
+    found = 0
+    for name, (_, body) in _functions().items():
+        if "tma_load_4d(" not in body:
+            continue
+        found += 1
+        # (in recon_sym3_kernel the load stands in a function that the first loop calls)
+        first = body.index("issue(p);" if "auto issue" in body else "tma_load_4d(")
+        assert body.index("pdl_begin()") < body.index("global_acquire_for_copies();") < first, name
+    assert found == 3
